@@ -1,0 +1,104 @@
+"""Spreading and interpolation by matrix products over strips of support starts.
+
+f32 results are compared with the f64 plan of the same tolerance, which uses
+the same window up to its Horner rows below 0.05 eps, so the difference is
+f32 rounding and at most a few such rows: window weights, strengths and sums
+carry a few units of 2^-24 each and the split products drop terms of 2^-22
+(together below 16 x 2^-23), and 0.2 eps stands for the rows. f64 results are
+compared with the direct sums at the reference's 20 eps (2D) and 32 eps (3D).
+"""
+
+import numpy as np
+import pytest
+
+from oracle import native
+
+pytestmark = pytest.mark.gpu
+
+F32_ROUNDING = 16 * 2.0**-23
+
+
+def points_of(rng, kind, count, fine):
+    """f32-exact points: uniform, crowded in one cell's neighbourhood, or on and beside the grid's edges."""
+    dims = len(fine)
+    p = rng.uniform(-np.pi, np.pi, (count, dims))
+    if kind == "crowded":
+        p[: count // 2] = rng.uniform(-0.2, 0.2, (count // 2, dims))
+    elif kind == "edges":
+        cell = 2.0 * np.pi / np.asarray(fine)
+        near = -np.pi + cell * rng.integers(-3, 4, (count, dims))
+        p = np.where(rng.random((count, dims)) < 0.5, np.remainder(near + np.pi, 2 * np.pi) - np.pi, p)
+        p[0] = np.nan  # out of reach: weighs zero
+    return p.astype(np.float32)
+
+
+def transform(w, kind, n_modes, eps, precision, batch, points, inputs, outputs):
+    import torch
+
+    real, cplx = ((torch.float32, torch.complex64) if precision == w.Precision.F32
+                  else (torch.float64, torch.complex128))
+    plan = w.NufftPlan(kind, w.NufftConfig(n_modes, eps, batch=batch, precision=precision))
+    out = torch.empty((batch, outputs), dtype=cplx, device="cuda")
+    plan.encode_gpu(torch.from_numpy(points).to("cuda", real), torch.from_numpy(inputs).to("cuda", cplx), out)
+    plan.synchronize()
+    return plan, out.cpu().numpy()
+
+
+def values(rng, batch, count):
+    return (rng.standard_normal((batch, count)) + 1j * rng.standard_normal((batch, count))).astype(np.complex64)
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("eps", [1e-4, 1e-5, 1e-6])
+@pytest.mark.parametrize("n_modes, count, spread, batch", [
+    ((16, 16, 16), 9, "uniform", 1),           # fewer points than a chunk
+    ((16, 16, 16), 40_000, "uniform", 1),      # one tile deep along z
+    ((21, 19, 33), 60_001, "crowded", 3),      # ragged tiles, parts of one tile
+    ((8, 40, 13), 30_003, "edges", 2),         # windows that wrap, a point out of reach
+])
+def test_f32_3d_differs_from_f64_by_rounding(kind, eps, n_modes, count, spread, batch):
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(11)
+    points = points_of(rng, spread, count, [2 * n for n in n_modes])
+    total = int(np.prod(n_modes))
+    inputs = values(rng, batch, count if kind == 1 else total)
+    outputs = total if kind == 1 else count
+    plan, got = transform(w, kind, n_modes, eps, w.Precision.F32, batch, points, inputs, outputs)
+    plan64, want = transform(w, kind, n_modes, eps, w.Precision.F64, batch, points, inputs, outputs)
+    # Support starts at exact cell boundaries may round to either side.
+    assert plan.kernel_width() == plan64.kernel_width()
+    if spread == "edges":
+        assert rel(got, want) < 32 * eps
+    else:
+        assert rel(got, want) < F32_ROUNDING + 0.2 * eps
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("eps", [1e-4, 1e-8, 1e-9, 1e-12, 1e-14])  # widths 5, 9, 10, 13, 15
+@pytest.mark.parametrize("n_modes, count, spread", [
+    ((40, 30), 5, "uniform"),
+    ((40, 30), 20_003, "crowded"),
+    ((9, 70), 6_001, "edges"),
+    ((12, 14, 10), 20_001, "uniform"),
+])
+def test_f64_matches_direct_sums(kind, eps, n_modes, count, spread):
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(12)
+    points = points_of(rng, spread, count, [2 * n for n in n_modes]).astype(np.float64)
+    total = int(np.prod(n_modes))
+    inputs = values(rng, 1, count if kind == 1 else total).astype(np.complex128)
+    _, got = transform(w, kind, n_modes, eps, w.Precision.F64, 1, points, inputs, total if kind == 1 else count)
+    reach = np.isfinite(points).all(axis=1)
+    if kind == 1:
+        want = native.direct_type1(points[reach], inputs[0][reach], n_modes)[0]
+    else:
+        want = np.zeros(count, dtype=np.complex128)
+        want[reach] = native.direct_type2(points[reach], inputs[0], n_modes)[0]
+    bound = max((20 if len(n_modes) == 2 else 32) * eps, 2e-13)  # 2e-13: rounding of the sums and the FFT
+    assert rel(got[0], want) < bound

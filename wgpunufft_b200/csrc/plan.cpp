@@ -484,6 +484,9 @@ void NufftPlan::configure_tiles() {
       sp.warp_segments = static_cast<const uint32_t*>(warp_segments_.get());
     }
   }
+  if (dim_ == 3 && precision_ == B200NUFFT_PRECISION_F32 && w >= kStripMinWidth && w <= kStripMaxWidth) {
+    spread_strip_layout(sp.pad, sp.strip_pitch0, sp.strip_pitch01);
+  }
   // Parts of at most kPartCap records (f64), fewer for small point sets so that
   // about four CTAs per SM have work. On one-cell bins holding eight or more
   // points per cell, consecutive records share their start: parts sized for
@@ -502,7 +505,10 @@ void NufftPlan::configure_tiles() {
   // 3D parts stay within the 2048 records that crowded tiles bucket in shared
   // memory; 1D and 2D f32 parts take up to 16384 records, so that a thread's
   // register runs can reach 64 records in crowded tiles.
-  const int64_t part_cap = dim_ == 3 ? 2048 : (precision_ == B200NUFFT_PRECISION_F32 ? 16384 : kPartCap);
+  // The f64 strips order at most kStripMaxRecords records.
+  const bool strips64 = dim_ == 2 && precision_ != B200NUFFT_PRECISION_F32 && w >= kStrip64MinWidth;
+  const int64_t part_cap = dim_ == 3 || strips64 ? kStripMaxRecords
+                                                 : (precision_ == B200NUFFT_PRECISION_F32 ? 16384 : kPartCap);
   cap = std::min<int64_t>(part_cap, std::max<int64_t>(256, (cap + 255) / 256 * 256));
   sp.part_cap = static_cast<int32_t>(cap);
   // The device sizes the parts from the points within reach (the others sort

@@ -24,12 +24,12 @@
 
 #include "device.h"
 #include "spread.h"
+#include "strips.cuh"
 
 namespace b200nufft {
 
 namespace {
 
-constexpr int kSpreadThreads = 256;
 
 // ---------------------------------------------------------------------------
 // Precision traits: coordinates, window, fixed-point accumulator.
@@ -437,10 +437,9 @@ __device__ __forceinline__ void flush_first_column(typename T::Word* acc, int pa
 // are taken in bin order. Points outside the fold reach or starting in
 // another tile are skipped.
 constexpr int kWarpRunBits = 5;
-constexpr int kWarpMaxRecords = 2048;  // the 3D part cap
+constexpr int kWarpMaxRecords = kStripMaxRecords;  // the 3D part cap
 constexpr int kWarpGroup = 8;          // records staged per warp at a time
 constexpr int kStageStride = 28;       // wx[8] wy[8] wz[8] re im base -
-constexpr int kSpreadWarps = kSpreadThreads / 32;
 
 template <int D, int W, typename T>
 __host__ __device__ constexpr bool warp_capable() {
@@ -716,96 +715,12 @@ __device__ void spread_warp3(const SpreadParams& sp, const PreparedWindow<3>* wi
   if (run >= 0) flush();
 }
 
-// 2D f64 tiles (windows of 5 taps or more, too wide for a thread's register
-// run) are spread by whole warps, one record at a time: lanes 0 .. 2w-1
-// evaluate one window tap each (axis a = lane / w), and lane l owns the
-// window cells u = l + 32 q (x = u mod w, y = u / w), summing a run of
-// records with one support start in f64 registers in record order. A run
-// reaches the 64-bit fixed-point tile once, when its start changes; the tile
-// of a part of at most 4096 records stays below 2^62 in every cell whatever
-// the runs, so the scale is the record-by-record one.
-template <int W>
-__device__ void spread_warp2_f64(const SpreadParams& sp, const double* points, const double2* sv,
-                                 const uint32_t* perm, const uint32_t* row_begin, const uint32_t* row_prefix,
-                                 int rows, const int* origin, uint32_t record_begin, uint32_t record_end,
-                                 unsigned long long* acc, int padded, double (*stage)[2][W], double scale_lo,
-                                 double scale_hi) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int R = (W * W + 31) / 32;
-  double ar[R], ai[R];
-#pragma unroll
-  for (int q = 0; q < R; ++q) ar[q] = ai[q] = 0.0;
-  int run_x = -1, run_y = 0;
-  const int pad0 = sp.pad[0];
-  auto flush = [&]() {
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int u = lane + 32 * q;
-      if (u < W * W) {
-        const int c = (run_y + u / W) * pad0 + run_x + u % W;
-        F64Traits::add(acc, padded, 0, c, ar[q]);
-        F64Traits::add(acc, padded, 1, c, ai[q]);
-      }
-      ar[q] = ai[q] = 0.0;
-    }
-  };
-  // Warp w spreads the consecutive records [warp_begin, warp_end).
-  const uint32_t n = record_end - record_begin;
-  const uint32_t per_warp = (n + kSpreadWarps - 1) / kSpreadWarps;
-  const uint32_t warp_begin = record_begin + min(n, per_warp * warp);
-  const uint32_t warp_end = record_begin + min(n, per_warp * (warp + 1));
-  const int axis = lane < W ? 0 : 1, tap = lane < W ? lane : lane - W;
-  double* my_tap = &stage[warp][axis][tap];
-  int row = 0;
-  // The next record's coordinates and point index are loaded one record
-  // ahead, and the strength as soon as its index is known.
-  double next_x = 0.0, next_y = 0.0;
-  uint32_t next_point = 0;
-  if (warp_begin < warp_end) {
-    const uint32_t slot = record_slot(warp_begin, row, row_begin, row_prefix, rows);
-    next_x = points[static_cast<int64_t>(slot) * 2];
-    next_y = points[static_cast<int64_t>(slot) * 2 + 1];
-    next_point = perm[slot];
-  }
-  for (uint32_t r = warp_begin; r < warp_end; ++r) {
-    const double x = next_x, y = next_y;
-    const double2 c = sv[next_point];
-    if (r + 1 < warp_end) {
-      const uint32_t slot = record_slot(r + 1, row, row_begin, row_prefix, rows);
-      next_x = points[static_cast<int64_t>(slot) * 2];
-      next_y = points[static_cast<int64_t>(slot) * 2 + 1];
-      next_point = perm[slot];
-    }
-    if (!F64Traits::in_reach(x) || !F64Traits::in_reach(y)) continue;
-    int32_t start[2];
-    double offset[2];
-    support_of64(x, sp.grid.axis64[0], sp.grid.half_width64, start[0], offset[0]);
-    support_of64(y, sp.grid.axis64[1], sp.grid.half_width64, start[1], offset[1]);
-    const int lx = wrap_start(start[0], sp.grid.axis[0].length) - origin[0];
-    const int ly = wrap_start(start[1], sp.grid.axis[1].length) - origin[1];
-    if (lx < 0 || lx >= sp.tile[0] || ly < 0 || ly >= sp.tile[1]) continue;  // another tile owns it
-    __syncwarp();  // the previous record's taps are read
-    if (lane < 2 * W) {
-      *my_tap = horner_weight(axis == 0 ? offset[0] : offset[1], tap, W, sp.grid.horner, sp.grid.horner_rows);
-    }
-    __syncwarp();
-    if (lx != run_x || ly != run_y) {
-      if (run_x >= 0) flush();
-      run_x = lx;
-      run_y = ly;
-    }
-    const double sr = (c.x * scale_lo) * scale_hi, si = (c.y * scale_lo) * scale_hi;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int u = lane + 32 * q;
-      if (u < W * W) {
-        const double weight = stage[warp][0][u % W] * stage[warp][1][u / W];
-        ar[q] = fma(sr, weight, ar[q]);
-        ai[q] = fma(si, weight, ai[q]);
-      }
-    }
-  }
-  if (run_x >= 0) flush();
+// Tiles that take the strips: 3D f32 tiles of enough records, all 2D f64
+// tiles of windows without register runs.
+template <int D, int W, typename T>
+__host__ __device__ constexpr bool strip_capable() {
+  if (sizeof(typename T::Real) == 8) return D == 2 && W >= kStrip64MinWidth;
+  return D == 3 && W >= kStripMinWidth && W <= kStripMaxWidth;
 }
 
 // 3D f64 tiles (windows of 5 taps or more) are spread by whole warps, one
@@ -880,13 +795,15 @@ __device__ void spread_warp3_f64(const SpreadParams& sp, const double* points, c
   }
 }
 
-// Resident CTAs per SM that the register budget is sized for: four for the
-// 2D f64 warp spreader, three for narrow windows without register runs, two for
-// register runs, other f64 windows and the 3D warp spreader.
+// Resident CTAs per SM that the register budget is sized for: three for narrow
+// windows without register runs, two for register runs, f64 windows, the 3D
+// warp spreader and the strips.
 template <int D, int W, typename T>
 __host__ __device__ constexpr int spread_min_blocks() {
-  if (D == 2 && sizeof(typename T::Real) == 8 && spread_run<D, W, T>() == 1 && W >= 5) return 4;
-  return (spread_run<D, W, T>() > 1 || sizeof(typename T::Real) == 8 || warp_capable<D, W, T>()) ? 2 : 3;
+  return (spread_run<D, W, T>() > 1 || sizeof(typename T::Real) == 8 || warp_capable<D, W, T>() ||
+          strip_capable<D, W, T>())
+             ? 2
+             : 3;
 }
 
 // Spreads part `part` of vector `b` (one CTA): the part's records into a
@@ -912,27 +829,33 @@ __device__ __forceinline__ void spread_part(
   const uint32_t total_parts = part_start[sp.tile_count];
   if (part >= total_parts) return;
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    // Last tile whose first part is at or below `part`.
-    int64_t low = 0, high = sp.tile_count - 1;
-    while (low < high) {
-      const int64_t mid = (low + high + 1) >> 1;
-      if (part_start[mid] <= part) low = mid; else high = mid - 1;
+  if (tid < 32) {
+    // Last tile whose first part is at or below `part`: a warp narrows the
+    // range 33-fold per step (dependent loads, on every CTA's critical path).
+    int64_t low = 0, count = sp.tile_count;  // the tile lies in [low, low + count)
+    while (count > 1) {
+      const int64_t step = (count + 32) / 33;
+      const int64_t probe = low + (tid + 1) * step;
+      const bool below = probe < low + count && part_start[probe] <= part;
+      const int passed = __popc(__ballot_sync(0xFFFFFFFFu, below));
+      count = min(step, count - passed * step);
+      low += passed * step;
     }
-    s_tile = low;
+    if (tid == 0) s_tile = low;
   }
   const int padded = sp.padded_cells;
   // The shared tile: dense (span = padded) or with the warp path's pitches.
   constexpr bool kWarpCapable = warp_capable<D, W, T>();
   const bool warp_path = kWarpCapable && sp.span > 0;
-  const int span = warp_path ? sp.span : padded;
-  {
+  int span = warp_path ? sp.span : padded;
+  auto clear_tile = [&]() {
     // Cleared 16 bytes at a time (the tile's words are a multiple of 16 bytes).
     static_assert(T::kWordsPerCell * sizeof(Word) % 16 == 0, "tile words clear in 16-byte units");
     uint4* acc16 = reinterpret_cast<uint4*>(acc);
     const int units = static_cast<int>(T::kWordsPerCell * sizeof(Word) / 16) * span;
     for (int c = tid; c < units; c += kSpreadThreads) acc16[c] = make_uint4(0u, 0u, 0u, 0u);
-  }
+  };
+  if constexpr (!strip_capable<D, W, T>()) clear_tile();
   __syncthreads();
   const int64_t tile = s_tile;
   const uint32_t part_in_tile = part - part_start[tile];
@@ -1008,8 +931,14 @@ __device__ __forceinline__ void spread_part(
   // fixed order within the run) and reach the fixed-point tile once per run,
   // which leaves that much headroom in the scale.
   constexpr int kRun = spread_run<D, W, T>();
-  __shared__ uint32_t sorted[kWarpCapable ? kWarpMaxRecords : 1];
-  __shared__ __align__(16) float stage[kWarpCapable ? kSpreadWarps : 1][kWarpGroup][kStageStride];
+  constexpr bool kStripCapable = strip_capable<D, W, T>();
+  __shared__ uint32_t sorted[kWarpCapable || kStripCapable ? kWarpMaxRecords : 1];
+  __shared__ uint32_t strip_start[kStripCapable ? kStripMax + 1 : 1];
+  __shared__ uint32_t strip_cell[kStripCapable ? kStripMax : 1];
+  constexpr bool kStrip64 = kStripCapable && sizeof(Real) == 8;
+  constexpr int kStageFloats = kStrip64 ? 2 * Strip64<W>::kDoubles
+                                        : (kStripCapable ? kStripFloats : (kWarpCapable ? kWarpGroup * kStageStride : 4));
+  __shared__ __align__(16) float stage[(kWarpCapable || kStripCapable ? kSpreadWarps : 1) * kStageFloats];
   const int tile_cells = sp.tile[0] * sp.tile[1] * sp.tile[2];
   const bool bucket = warp_path && record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
                       (tile_cells + 1) * kSpreadWarps <= T::kWordsPerCell * span &&
@@ -1020,27 +949,64 @@ __device__ __forceinline__ void spread_part(
   const typename T::Complex* sv = strengths + static_cast<int64_t>(b) * point_count;
 
   int row = 0;
-  if constexpr (kWarpCapable) {
-    if (warp_path) {
-      spread_warp3<W>(sp, static_cast<const PreparedWindow<3>*>(windows), sv, perm, row_begin, row_prefix, rows,
-                      origin, record_begin, record_end, bucket, acc, span, sorted, stage,
-                      T::exponent(max_bits[b]), S);
+  // Tiles with enough records per start cell take the tensor-core strips.
+  bool strip_path = false;
+  int pitch0 = warp_path ? sp.pitch0 : sp.pad[0];
+  int pitch01 = warp_path ? sp.pitch01 : sp.pad[0] * sp.pad[1];
+  if constexpr (kStripCapable && !kStrip64) {
+    constexpr int kS = 9 - W;
+    const int strips = ((sp.tile[0] + kStripX - 1) / kStripX) * ((sp.tile[1] + kS - 1) / kS) *
+                       ((sp.tile[2] + kS - 1) / kS);
+    strip_path = sp.strip_pitch0 > 0 && strips <= kStripMax && record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
+                 (strips * kStripX + 1) * kSpreadWarps <= T::kWordsPerCell * span &&
+                 tile_total * static_cast<uint32_t>(strip_cells_per_record(W)) >= static_cast<uint32_t>(tile_cells);
+    if (strip_path) {
+      // A warp's register sums hold at most 2^8 + 2^6 records of magnitude
+      // below 2^29: below 2^38, which add_split takes.
+      S = T::exponent(max_bits[b]) - 1;
+      pitch0 = sp.strip_pitch0;
+      pitch01 = sp.strip_pitch01;
+      span = pitch01 * sp.pad[2];
+      spread_strips3<W>(sp, static_cast<const PreparedWindow<3>*>(windows), sv, perm, row_begin, row_prefix, rows,
+                        origin, record_begin, record_end, acc, span, pitch0, pitch01,
+                        StripShared{sorted, strip_start, strip_cell, stage}, T::power_of_two(S / 2),
+                        T::power_of_two(S - S / 2));
+    } else {
+      clear_tile();
+      __syncthreads();
     }
   }
-  constexpr bool kWarp64 = D >= 2 && sizeof(Real) == 8 && kRun == 1 && W >= 5;
-  __shared__ double stage64[kWarp64 ? kSpreadWarps : 1][kWarp64 ? D : 1][kWarp64 ? W : 1];
-  if constexpr (kWarp64 && D == 2) {
-    spread_warp2_f64<W>(sp, reinterpret_cast<const double*>(points), reinterpret_cast<const double2*>(sv), perm,
-                        row_begin, row_prefix, rows, origin, record_begin, record_end,
-                        reinterpret_cast<unsigned long long*>(acc), padded, stage64, scale_lo, scale_hi);
+  if constexpr (kWarpCapable) {
+    if (warp_path && !strip_path) {
+      spread_warp3<W>(sp, static_cast<const PreparedWindow<3>*>(windows), sv, perm, row_begin, row_prefix, rows,
+                      origin, record_begin, record_end, bucket, acc, span, sorted,
+                      reinterpret_cast<float(*)[kWarpGroup][kStageStride]>(stage), T::exponent(max_bits[b]), S);
+    }
   }
-  if constexpr (kWarp64 && D == 3) {
+  if constexpr (kStrip64) {
+    // The window's Horner table in shared memory: per row the even taps, then the odd ones.
+    using L = Strip64<W>;
+    __shared__ __align__(16) double table[L::kRows * 2 * L::kTaps];
+    for (int i = tid; i < L::kRows * 2 * L::kTaps; i += kSpreadThreads) {
+      const int tap = 2 * (i % L::kTaps) + (i / L::kTaps) % 2;
+      const int r = i / (2 * L::kTaps) - (L::kRows - sp.grid.horner_rows);  // leading rows may be missing: zero
+      table[i] = tap < W && r >= 0 ? sp.grid.horner[r * W + tap] : 0.0;
+    }
+    strip_path = true;
+    spread_strips2_f64<W>(sp, reinterpret_cast<const double2*>(points), reinterpret_cast<const double2*>(sv), perm,
+                          row_begin, row_prefix, rows, origin, record_begin, record_end,
+                          reinterpret_cast<unsigned long long*>(acc), padded,
+                          StripShared{sorted, strip_start, strip_cell, stage}, table, scale_lo, scale_hi);
+  }
+  constexpr bool kWarp64 = D == 3 && sizeof(Real) == 8 && W >= 5;
+  __shared__ double stage64[kWarp64 ? kSpreadWarps : 1][kWarp64 ? D : 1][kWarp64 ? W : 1];
+  if constexpr (kWarp64) {
     spread_warp3_f64<W>(sp, reinterpret_cast<const double*>(points), reinterpret_cast<const double2*>(sv), perm,
                         row_begin, row_prefix, rows, origin, record_begin, record_end,
                         reinterpret_cast<unsigned long long*>(acc), padded, stage64, scale_lo, scale_hi);
   }
-  if constexpr (kRun == 1 && !kWarp64) {
-    for (uint32_t r = record_begin + tid; !warp_path && r < record_end; r += kSpreadThreads) {
+  if constexpr (kRun == 1 && !kWarp64 && !kStrip64) {
+    for (uint32_t r = record_begin + tid; !warp_path && !strip_path && r < record_end; r += kSpreadThreads) {
       int local_start[D];
       Real w[D][W];
       typename T::Complex s;
@@ -1189,38 +1155,41 @@ __device__ __forceinline__ void spread_part(
   }
   __syncthreads();
   typename T::Complex* out = scratch + (static_cast<int64_t>(part) * batch + b) * padded;
-  if (warp_path) {
-    // The thread's cells c = tid + k kSpreadThreads: (x, y, z) stepped by
-    // the stride's own coordinates with one carry per axis, not divided.
-    const int pad0 = sp.pad[0], pad1 = sp.pad[1], pad01 = sp.pad[0] * sp.pad[1];
-    int z = tid / pad01, y = (tid - z * pad01) / pad0;
-    int x = tid - z * pad01 - y * pad0;
-    const int step_z = kSpreadThreads / pad01, step_y = (kSpreadThreads - step_z * pad01) / pad0;
-    const int step_x = kSpreadThreads - step_z * pad01 - step_y * pad0;
+  // The strips' low words are signed sums, below 2^24 as the high words of
+  // all but extreme cells: one rounding.
+  const float down_lo = T::kPreparedWindows ? ldexpf(1.0f, -S / 2) : 0.0f;
+  const float down_hi = T::kPreparedWindows ? ldexpf(1.0f, -S - (-S / 2)) : 0.0f;
+  auto value = [&](int which, int at) {
+    if constexpr (kStripCapable && !kStrip64) {
+      if (strip_path) {
+        const float lo = static_cast<float>(static_cast<int32_t>(acc[(2 * which) * span + at]));
+        const float hi = static_cast<float>(static_cast<int32_t>(acc[(2 * which + 1) * span + at]));
+        return fmaf(hi, 65536.0f, lo) * down_lo * down_hi;
+      }
+    }
+    return T::value(acc, span, which, at, S);
+  };
+  if (warp_path || (strip_path && !kStrip64)) {
+    // Cells' planes and rows from reciprocals (exact: cells and pitches below 2^16).
+    const uint32_t pad0 = sp.pad[0], pad01 = sp.pad[0] * sp.pad[1];
+    const uint32_t per01 = 0xFFFFFFFFu / pad01 + 1u, per0 = 0xFFFFFFFFu / pad0 + 1u;
+    const int slack0 = pitch0 - sp.pad[0], slack01 = pitch01 - pitch0 * sp.pad[1];
+#pragma unroll 4
     for (int c = tid; c < padded; c += kSpreadThreads) {
-      const int at = x + y * sp.pitch0 + z * sp.pitch01;
+      const uint32_t z = __umulhi(c, per01), row = __umulhi(c, per0);
+      const int at = c + static_cast<int>(row) * slack0 + static_cast<int>(z) * slack01;
       typename T::Complex v;
-      v.x = T::value(acc, span, 0, at, S);
-      v.y = T::value(acc, span, 1, at, S);
+      v.x = value(0, at);
+      v.y = value(1, at);
       out[c] = v;
-      x += step_x;
-      y += step_y;
-      z += step_z;
-      if (x >= pad0) {
-        x -= pad0;
-        ++y;
-      }
-      if (y >= pad1) {
-        y -= pad1;
-        ++z;
-      }
     }
     return;
   }
+#pragma unroll 4
   for (int c = tid; c < padded; c += kSpreadThreads) {
     typename T::Complex v;
-    v.x = T::value(acc, padded, 0, c, S);
-    v.y = T::value(acc, padded, 1, c, S);
+    v.x = value(0, c);
+    v.y = value(1, c);
     out[c] = v;
   }
 }
@@ -1582,7 +1551,8 @@ void fold_any(const SpreadParams& sp, int batch, const Complex* scratch, const u
 
 template <int D, int W, typename T>
 void launch_spread_width(const SpreadParams& sp, const SpreadLaunchT<T>& l, cudaStream_t stream) {
-  const int span = warp_capable<D, W, T>() && sp.span > 0 ? sp.span : sp.padded_cells;
+  int span = warp_capable<D, W, T>() && sp.span > 0 ? sp.span : sp.padded_cells;
+  if (strip_capable<D, W, T>()) span = std::max(span, sp.strip_pitch01 * sp.pad[2]);
   const size_t smem = static_cast<size_t>(T::kWordsPerCell) * span * sizeof(typename T::Word);
   auto kernel = spread_tiles_kernel<D, W, T>;
   check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1813,7 +1783,8 @@ void spread_fold(const SpreadParams& sp, const SpreadLaunch& l, cudaStream_t str
 size_t spread_shared_bytes(const SpreadParams& sp) {
   const int w = sp.grid.width;
   const bool warp = sp.grid.dimensions == 3 && w >= kWarpMinWidth && w <= kWarpMaxWidth && sp.span > 0;
-  return static_cast<size_t>(F32Traits::kWordsPerCell) * (warp ? sp.span : sp.padded_cells) * sizeof(uint32_t);
+  const int span = std::max(warp ? sp.span : sp.padded_cells, sp.strip_pitch01 * sp.pad[2]);
+  return static_cast<size_t>(F32Traits::kWordsPerCell) * span * sizeof(uint32_t);
 }
 
 void spread_count_parts(const SpreadParams& sp, const uint32_t* offsets, uint32_t* parts,
@@ -1844,6 +1815,25 @@ void spread_execute(const SpreadParams& sp, const SpreadLaunch& l, cudaStream_t 
                              l.perm,     l.offsets,          l.part_start,  l.part_upper_bound,
                              l.max_bits, l.scratch,          l.candidates,  l.fine, l.valid_mask};
   spread_execute_impl<F32Traits>(sp, t, stream, timer);
+}
+
+void spread_strip_layout(const int32_t pad[3], int32_t& pitch0, int32_t& pitch01) {
+  int best = 33;
+  for (int d0 = 0; d0 < 2; ++d0) {
+    for (int d1 = 0; d1 < 8; ++d1) {
+      const int p0 = pad[0] + d0, p01 = p0 * pad[1] + d1;
+      int banks[32] = {};
+      for (int y = 0; y < 8; ++y) {
+        for (int z = 0; z < 8; z += 2) ++banks[(y * p0 + z * p01) & 31];
+      }
+      const int most = *std::max_element(banks, banks + 32);
+      if (most < best) {
+        best = most;
+        pitch0 = p0;
+        pitch01 = p01;
+      }
+    }
+  }
 }
 
 bool spread_warp_layout(int width, const int32_t pad[3], int32_t& pitch0, int32_t& pitch01,

@@ -49,6 +49,10 @@ struct SpreadParams {
   int32_t pitch01;
   int32_t span;
   const uint32_t* warp_segments;
+  // 3D f32 plans of widths kStripMinWidth..kStripMaxWidth: pitches of the
+  // padded tile under the tensor-core strips (spread_strip_layout).
+  int32_t strip_pitch0;
+  int32_t strip_pitch01;
   // 3D plans of 16 x 16 x (4 k)-cell tiles whose cells' candidate lists are,
   // along every axis, ordered parts of the list of their tile's first cell
   // (checked on the host): single vectors fold per destination tile
@@ -82,6 +86,21 @@ constexpr uint32_t kSegmentValid = 0x80000000u;
 // false when no pitch reaches the warp_rounds(width) rounds.
 bool spread_warp_layout(int width, const int32_t pad[3], int32_t& pitch0, int32_t& pitch01,
                         uint32_t* table);
+
+// Window widths that crowded 3D f32 tiles spread on the tensor cores: the
+// strips hold 9 - w support starts along y and z, so w = 8 would leave one;
+// below 5 the w^3 adds of a point cost less until tiles hold several points
+// per cell (96^3 modes, uniform, w 4: 261 us per-point adds against 310 at 1/4
+// point per cell, 464 against 466 at 1/2), and the per-point kernel keeps
+// three CTAs per SM without them.
+constexpr int kStripMinWidth = 5;
+constexpr int kStripMaxWidth = 7;
+// 2D f64 windows without register runs (spread_run) always take the strips.
+constexpr int kStrip64MinWidth = 5;
+constexpr int kStripMaxRecords = 2048;  // records of a part under the strips, at most
+// Pitches of the padded tile (pad[a] cells, some slack allowed) that spread
+// a strip's flush, 8 rows x 4 even planes per warp, over the most banks.
+void spread_strip_layout(const int32_t pad[3], int32_t& pitch0, int32_t& pitch01);
 
 struct SpreadLaunch {
   const float* points;    // coordinates in bin (slot) order
