@@ -30,6 +30,15 @@ struct InterpLaunch64 {
 
 void interpolate_execute(const GridParams& g, const InterpLaunch& launch, cudaStream_t stream);
 
+// Interpolation by matrix products over strips (interp_strips.cu): 2D and 3D
+// plans whose points (and windows, permutation) are ordered by bins of the
+// sides 2^shift[a] of their support starts.
+// Whether a plan's point set takes them (the rest gathers per point).
+bool interp_strips_chosen(int dimensions, bool f64, int width, int64_t points, int64_t cells);
+void interp_strip_shifts(bool f64, int32_t shift[3]);
+void interp_strips_execute(const GridParams& g, const InterpLaunch& launch, cudaStream_t stream);
+void interp_strips_execute64(const GridParams& g, const InterpLaunch64& launch, cudaStream_t stream);
+
 // Work items of the 2D bin interpolation kernels: the slots of every bin in
 // parts of at most kInterpPartSlots, so that a bin holding many points
 // (clustered points) is served by many CTAs instead of one. part_bin[p] is
@@ -77,10 +86,4 @@ void interpolate_execute64(const GridParams& g, const InterpLaunch64& launch, cu
 // output[b][i] = staged[inverse[i] * stride + b] for b < batch, i < count.
 void unpermute_values(const float2* staged, int64_t stride, const uint32_t* inverse, int64_t count, int batch,
                       float2* output, cudaStream_t stream);
-// 2D f64 plans on 4 x 4-cell bins: each bin's grid region staged in shared
-// memory (same sums, bit for bit, as interpolate_execute64).
-bool interpolate_region64_supported(const GridParams& g);
-void interpolate_region64_execute(const GridParams& g, const InterpLaunch64& launch, const uint32_t* offsets,
-                                  uint64_t bins, const InterpParts& parts, cudaStream_t stream);
-
 }  // namespace b200nufft

@@ -1,0 +1,352 @@
+// Type-2 interpolation by small matrix products (mma.sync): 2D and 3D plans
+// whose points are ordered by strips of support starts.
+//
+// set_points orders the points by (z strip, y strip, x start), the strips a
+// few cells wide (interp_strip_shifts). A warp takes 32 consecutive points and
+// serves them in groups of one strip whose starts lie within kSpan cells of x.
+// For a group, every plane z and every block of 4 columns,
+//   T[point, x] = sum_y wy[point, y] G[z, y, x]
+// is a product with the strip's rows as the contracted index (f32: 8 rows,
+// m16n8k8 on tf32 high and low parts, smallest products first, from zero; f64:
+// m8n8k4), whose right operand, the grid values, is loaded once for 32 points
+// straight into fragments; each point then adds wx wz T to its sum. The
+// gather of w^d cells per point becomes a few loads per point.
+//
+// A point's sum depends on its own window alone: rows and columns outside
+// it weigh zero, blocks and rows are fixed by the grid, so the bits do not
+// depend on the group, the batch or the other points.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "device.h"
+#include "interp.h"
+#include "mma.cuh"
+
+namespace b200nufft {
+
+namespace {
+
+constexpr int kSpan = 16;  // x starts of a group, at most
+
+// Strip sides (log2) along y and z: the rows a strip's windows reach fill the
+// contracted index (8 rows in f32, multiples of 4 in f64); z strips of 4.
+template <int W, bool F64>
+struct Strip {
+  static constexpr int kShiftY = F64 ? 2 : 1;
+  static constexpr int kShiftZ = 2;
+  static constexpr int kRows = F64 ? ((1 << kShiftY) + W - 1 + 3) / 4 * 4 : 8;
+  static constexpr int kPitchY = kRows % 8 == 0 ? kRows + 4 : kRows;  // conflict-free fragment reads
+  static constexpr int kPitchX = W | 1;
+  // z weights at their place among the planes of the strip, zeros around them.
+  static constexpr int kPlanes = (1 << kShiftZ) + W - 1;
+  static constexpr int kPitchZ = kPlanes | 1;
+};
+
+template <int D, int W, typename Real>
+struct WarpStage {
+  using S = Strip<W, sizeof(Real) == 8>;
+  Real wy[32 * S::kPitchY];
+  Real wx[32 * S::kPitchX];
+  Real wz[D == 3 ? 32 * S::kPitchZ : 1];
+};
+
+struct F32Strips {
+  using Real = float;
+  using Complex = float2;
+  static constexpr int kWarps = 4;
+};
+struct F64Strips {
+  using Real = double;
+  using Complex = double2;
+  static constexpr int kWarps = 2;
+};
+
+template <int D, int W, typename T>
+__global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
+    GridParams grid, const typename T::Real* __restrict__ points, const void* __restrict__ windows, int64_t count,
+    const uint32_t* __restrict__ perm, const typename T::Complex* __restrict__ fine, int batch,
+    typename T::Complex* __restrict__ output) {
+  using Real = typename T::Real;
+  using Complex = typename T::Complex;
+  constexpr bool F64 = sizeof(Real) == 8;
+  using S = Strip<W, F64>;
+  constexpr int K = F64 ? S::kRows / 4 : 1;  // products along the rows
+  __shared__ __align__(16) WarpStage<D, W, Real> stages[T::kWarps];
+  // The f64 Horner table, bottom-aligned (EsHornerTable::fit drops leading rows that vanish).
+  constexpr int kHorner = W + 3 < kMaxHornerCoefficients ? W + 3 : kMaxHornerCoefficients;
+  __shared__ double table[F64 ? kHorner * W : 1];
+  if constexpr (F64) {
+    const int missing = (kHorner - grid.horner_rows) * W;
+    for (int i = threadIdx.x; i < kHorner * W; i += T::kWarps * 32) {
+      table[i] = i >= missing ? grid.horner[i - missing] : 0.0;
+    }
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t first = (static_cast<int64_t>(blockIdx.x) * T::kWarps + warp) * 32;
+  if (first >= count) return;
+  WarpStage<D, W, Real>& st = stages[warp];
+  const int n0 = grid.axis[0].length, n1 = grid.axis[1].length, n2 = D == 3 ? grid.axis[2].length : 1;
+  const int64_t plane_cells = D == 3 ? static_cast<int64_t>(n0) * n1 : 0;
+
+  // Lane = point: its starts, and its windows staged.
+  const int64_t slot = first + lane;
+  const bool exists = slot < count;
+  int start[3] = {0, 0, 0};
+  bool reach = false;
+  uint32_t point = 0;
+  {
+    Real w[W];
+    auto place = [&](int a) {
+      if (a == 1) {
+        Real* row = st.wy + lane * S::kPitchY;
+#pragma unroll
+        for (int j = 0; j < S::kRows; ++j) row[j] = Real(0);
+        row += start[1] & ((1 << S::kShiftY) - 1);
+#pragma unroll
+        for (int j = 0; j < W; ++j) row[j] = w[j];
+      } else if (a == 0) {
+        Real* row = st.wx + lane * S::kPitchX;
+#pragma unroll
+        for (int j = 0; j < W; ++j) row[j] = w[j];
+      } else {
+        Real* row = st.wz + lane * S::kPitchZ;
+#pragma unroll
+        for (int j = 0; j < S::kPlanes; ++j) row[j] = Real(0);
+        row += start[2] & ((1 << S::kShiftZ) - 1);
+#pragma unroll
+        for (int j = 0; j < W; ++j) row[j] = w[j];
+      }
+    };
+    if (exists) point = __ldg(perm + slot);
+    if constexpr (!F64) {
+      PreparedWindow<D> win{};
+      win.start[0] = -1;
+      if (exists) win = static_cast<const PreparedWindow<D>*>(windows)[slot];
+      reach = win.start[0] >= 0;
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        start[a] = reach ? win.start[a] : 0;
+        horner32_window<W>(win.offset[a], grid.horner32, w);
+        place(a);
+      }
+    } else {
+      double p[D];
+#pragma unroll
+      for (int a = 0; a < D; ++a) p[a] = exists ? points[slot * D + a] : 0.0;
+      reach = exists;
+#pragma unroll
+      for (int a = 0; a < D; ++a) reach = reach && in_fold_reach64(p[a]);
+#pragma unroll
+      for (int a = 0; a < D; ++a) {
+        int32_t s = 0;
+        double offset = 0.0;
+        if (reach) support_of64(p[a], grid.axis64[a], grid.half_width64, s, offset);
+        start[a] = wrap_start(s, grid.axis[a].length);
+        const double local = 2.0 * offset + static_cast<double>(W - 1);
+        const bool inside = fabs(local) <= 1.0;
+#pragma unroll
+        for (int j = 0; j < W; ++j) w[j] = 0.0;
+#pragma unroll 4
+        for (int r = 0; r < kHorner; ++r) {
+#pragma unroll
+          for (int j = 0; j < W; ++j) w[j] = fma(w[j], local, table[r * W + j]);
+        }
+#pragma unroll
+        for (int j = 0; j < W; ++j) w[j] = inside ? w[j] : 0.0;
+        place(a);
+      }
+    }
+  }
+  if (exists && !reach) {
+    Complex zero;
+    zero.x = zero.y = Real(0);
+    for (int b = 0; b < batch; ++b) output[static_cast<int64_t>(b) * count + point] = zero;
+  }
+  __syncwarp();
+
+  // Fragments: lane (g, t) holds rows (points) 8 m + g, and columns
+  // x = 4 n + t (real and imaginary part) of the products.
+  const int g = lane >> 2, t = lane & 3;
+  int px[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    px[m] = __shfl_sync(0xFFFFFFFFu, start[0], 8 * m + g);
+  }
+  const uint32_t destination = __shfl_sync(0xFFFFFFFFu, point, 8 * t + g);
+  // Left operands (row weights) of the 32 points.
+  [[maybe_unused]] uint32_t ah[2][4], al[2][4];
+  [[maybe_unused]] double a64[4][K];
+  if constexpr (!F64) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const float* row = reinterpret_cast<const float*>(st.wy) + (16 * m + g) * S::kPitchY + t;
+      split_tf32(row[0], ah[m][0], al[m][0]);
+      split_tf32(row[8 * S::kPitchY], ah[m][1], al[m][1]);
+      split_tf32(row[4], ah[m][2], al[m][2]);
+      split_tf32(row[8 * S::kPitchY + 4], ah[m][3], al[m][3]);
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) a64[m][k] = st.wy[(8 * m + g) * S::kPitchY + 4 * k + t];
+    }
+  }
+  const int strip_y = start[1] >> S::kShiftY, strip_z = D == 3 ? start[2] >> S::kShiftZ : 0;
+  unsigned todo = __ballot_sync(0xFFFFFFFFu, reach);
+  while (todo != 0u) {
+    const int leader = __ffs(todo) - 1;
+    const int lx = __shfl_sync(0xFFFFFFFFu, start[0], leader);
+    const int ly = __shfl_sync(0xFFFFFFFFu, strip_y, leader);
+    const int lz = D == 3 ? __shfl_sync(0xFFFFFFFFu, strip_z, leader) : 0;
+    const bool mine = ((todo >> lane) & 1u) && strip_y == ly && strip_z == lz && start[0] >= lx &&
+                      start[0] < lx + kSpan;
+    const unsigned members = __ballot_sync(0xFFFFFFFFu, mine);
+    todo &= ~members;
+    const int hx = __reduce_max_sync(0xFFFFFFFFu, mine ? start[0] : lx) + W - 1;
+    int z_lo = 0, z_hi = 0;
+    if (D == 3) {
+      z_lo = __reduce_min_sync(0xFFFFFFFFu, mine ? start[2] : 0x7FFFFFFF);
+      z_hi = __reduce_max_sync(0xFFFFFFFFu, mine ? start[2] : 0) + W - 1;
+    }
+    // Grid rows of the lane's contracted indexes, as element offsets of a plane.
+    int64_t row_at[F64 ? K : 2];
+#pragma unroll
+    for (int k = 0; k < (F64 ? K : 2); ++k) {
+      int y = (ly << S::kShiftY) + 4 * k + t;
+      while (y >= n1) y -= n1;
+      row_at[k] = static_cast<int64_t>(y) * n0;
+    }
+    for (int b = 0; b < batch; ++b) {
+      const Real* const values = reinterpret_cast<const Real*>(fine + static_cast<int64_t>(b) * grid.fine_count) + (g & 1);
+      Complex v[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) v[m].x = v[m].y = Real(0);
+      for (int n = lx >> 2; n <= hx >> 2; ++n) {
+        int column = 4 * n + (g >> 1);
+        column = column >= n0 ? column - n0 : column;
+        Real wx[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const int i = 4 * n + t - px[m];
+          wx[m] = static_cast<unsigned>(i) < static_cast<unsigned>(W) ? st.wx[(8 * m + g) * S::kPitchX + i] : Real(0);
+        }
+        const Real* const weights_z = st.wz + g * S::kPitchZ - (lz << S::kShiftZ);
+#pragma unroll 2
+        for (int z = z_lo; z <= z_hi; ++z) {
+          const int64_t plane = D == 3 ? static_cast<int64_t>(z >= n2 ? z - n2 : z) * plane_cells : 0;
+          const Real* const at = values + 2 * (plane + column);
+          Real weight[4];
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            weight[m] = wx[m];
+            if (D == 3) weight[m] *= weights_z[8 * m * S::kPitchZ + z];
+          }
+          if constexpr (!F64) {
+            uint32_t bh0, bl0, bh1, bl1;
+            split_tf32(__ldg(at + 2 * row_at[0]), bh0, bl0);
+            split_tf32(__ldg(at + 2 * row_at[1]), bh1, bl1);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+              mma_tf32(d, al[m], bh0, bh1);
+              mma_tf32(d, ah[m], bl0, bl1);
+              mma_tf32(d, ah[m], bh0, bh1);
+              v[2 * m] = cfma(make_float2(d[0], d[1]), weight[2 * m], v[2 * m]);
+              v[2 * m + 1] = cfma(make_float2(d[2], d[3]), weight[2 * m + 1], v[2 * m + 1]);
+            }
+          } else {
+            double2 d[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) d[m] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+              const double value = __ldg(at + 2 * row_at[k]);
+#pragma unroll
+              for (int m = 0; m < 4; ++m) mma_f64(d[m], a64[m][k], value);
+            }
+#pragma unroll
+            for (int m = 0; m < 4; ++m) v[m] = cfma(d[m], weight[m], v[m]);
+          }
+        }
+      }
+      // The columns' sums; lane t keeps point 8 t + g.
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        v[m].x += __shfl_xor_sync(0xFFFFFFFFu, v[m].x, 1);
+        v[m].y += __shfl_xor_sync(0xFFFFFFFFu, v[m].y, 1);
+        v[m].x += __shfl_xor_sync(0xFFFFFFFFu, v[m].x, 2);
+        v[m].y += __shfl_xor_sync(0xFFFFFFFFu, v[m].y, 2);
+      }
+      const Complex e = t == 0 ? v[0] : (t == 1 ? v[1] : (t == 2 ? v[2] : v[3]));
+      if ((members >> (8 * t + g)) & 1u) output[static_cast<int64_t>(b) * count + destination] = e;
+    }
+  }
+}
+
+template <int D, int W, typename T>
+void launch_width(const GridParams& g, const typename T::Real* points, const void* windows, int64_t count,
+                  const uint32_t* perm, const typename T::Complex* fine, int batch, typename T::Complex* output,
+                  cudaStream_t stream) {
+  const unsigned blocks = static_cast<unsigned>((count + 32 * T::kWarps - 1) / (32 * T::kWarps));
+  interp_strips_kernel<D, W, T><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count, perm, fine, batch,
+                                                                       output);
+  note_launch();
+}
+
+}  // namespace
+
+bool interp_strips_chosen(int dimensions, bool f64, int width, int64_t points, int64_t cells) {
+  if (f64) {
+    if (width < 5) return false;
+    return dimensions == 2 || (dimensions == 3 && points * (width < 12 ? 6 : 12) >= cells);
+  }
+  return dimensions == 3 && ((width == 6 && points * 3 >= cells) || (width == 7 && points * 4 >= cells));
+}
+
+void interp_strip_shifts(bool f64, int32_t shift[3]) {
+  shift[0] = 0;
+  shift[1] = f64 ? Strip<kMaxWidth, true>::kShiftY : Strip<7, false>::kShiftY;
+  shift[2] = Strip<7, false>::kShiftZ;
+}
+
+void interp_strips_execute(const GridParams& g, const InterpLaunch& l, cudaStream_t stream) {
+  if (l.point_count == 0) return;
+  auto launch = [&](auto kernel) {
+    kernel(g, l.points, l.windows, l.point_count, l.perm, l.fine, l.batch, l.output, stream);
+  };
+  switch (g.width) {
+    case 6: launch(launch_width<3, 6, F32Strips>); break;
+    default: launch(launch_width<3, 7, F32Strips>); break;
+  }
+}
+
+void interp_strips_execute64(const GridParams& g, const InterpLaunch64& l, cudaStream_t stream) {
+  if (l.point_count == 0) return;
+  auto launch = [&](auto kernel2, auto kernel3) {
+    (g.dimensions == 2 ? kernel2 : kernel3)(g, l.points, nullptr, l.point_count, l.perm, l.fine, l.batch, l.output,
+                                            stream);
+  };
+  switch (g.width) {
+#define B200NUFFT_STRIPS_CASE(WIDTH) \
+  case WIDTH: launch(launch_width<2, WIDTH, F64Strips>, launch_width<3, WIDTH, F64Strips>); break;
+    B200NUFFT_STRIPS_CASE(5)
+    B200NUFFT_STRIPS_CASE(6)
+    B200NUFFT_STRIPS_CASE(7)
+    B200NUFFT_STRIPS_CASE(8)
+    B200NUFFT_STRIPS_CASE(9)
+    B200NUFFT_STRIPS_CASE(10)
+    B200NUFFT_STRIPS_CASE(11)
+    B200NUFFT_STRIPS_CASE(12)
+    B200NUFFT_STRIPS_CASE(13)
+    B200NUFFT_STRIPS_CASE(14)
+    B200NUFFT_STRIPS_CASE(15)
+    default:
+    B200NUFFT_STRIPS_CASE(16)
+#undef B200NUFFT_STRIPS_CASE
+  }
+}
+
+}  // namespace b200nufft

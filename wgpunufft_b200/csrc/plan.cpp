@@ -713,11 +713,9 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       tc2_part_upper_bound_ = tiles + chunk_bound / kTi2ChunksPerPart + 1;
       tc2_vector_max_.reserve(static_cast<size_t>(std::max<int64_t>(batch_, 1)) * sizeof(uint32_t), "vector maxima");
     }
-    // 3D type 2: the interpolation takes the points in the order of their
-    // support starts' (z, y) rows and 8-cell segments of x, so that a warp's
-    // 32 points gather from few grid rows; only that order is sorted here
-    // (its permutation kept), the reference's bins when they are asked for.
-    rows_order_ = type_ == 2 && dim_ == 3 && count > 0;
+    // The interpolation's own order (rows_grid) is sorted here and its
+    // permutation kept; the reference's bins are sorted when they are asked for.
+    rows_order_ = interp_rows_order() && count > 0;
     if (rows_order_) {
       uint64_t stride = 0;
       const GridParams rows = rows_grid(&stride);
@@ -749,7 +747,7 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
                                        "point slots");
       invert_permutation(perm_, count, static_cast<uint32_t*>(inverse), stream);
     }
-    if (type_ == 2 && dim_ == 2) prepare_interp_parts(offsets, stream);
+    if (type_ == 2 && dim_ == 2 && !rows_order_) prepare_interp_parts(offsets, stream);
   } else {
     const double* points64 = static_cast<const double*>(points);
     if (precision_ == B200NUFFT_PRECISION_DF64 && count > 0) {
@@ -757,8 +755,8 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       df64_to_f64(static_cast<const float*>(points), count * dim_, converted, stream);
       points64 = converted;
     }
-    // 3D type 2: the interpolation's row order alone, as for f32 plans.
-    rows_order_ = type_ == 2 && dim_ == 3 && count > 0;
+    // The interpolation's order alone, as for f32 plans.
+    rows_order_ = interp_rows_order() && count > 0;
     if (rows_order_) {
       uint64_t stride = 0;
       const GridParams rows = rows_grid(&stride);
@@ -775,10 +773,6 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
     }
     double* sorted = static_cast<double*>(sorted_points_.reserve(sorted_bytes, "sorted coordinates"));
     gather_sorted_points64(points64, interp_perm(), count, dim_, sorted, stream, &timer_);
-    if (type_ == 2 && dim_ == 2) {
-      StageScope scope(&timer_, kStageBinOffsets, stream);
-      prepare_interp_parts(offsets, stream);
-    }
   }
   if (type_ == 1) {
     configure_tiles();
@@ -987,6 +981,19 @@ void NufftPlan::execute_f32(int batch, const void* input, void* output, uint64_t
       tc_interp_execute(tc2_grid_, t, stream);
       return;
     }
+    if (rows_order_ && interp_strips()) {
+      InterpLaunch l;
+      l.points = static_cast<const float*>(sorted_points_.get());
+      l.windows = windows_.get();
+      l.point_count = point_count_;
+      l.perm = interp_perm();
+      l.fine = fine;
+      l.batch = batch;
+      l.output = static_cast<float2*>(output);
+      StageScope scope(&timer_, kStageInterpolation, stream);
+      interp_strips_execute(grid_, l, stream);
+      return;
+    }
     if (dim_ == 2 && batch >= kInterpBinsMinBatch && interpolate_bins_supported(grid_)) {
       InterpBinsLaunch b;
       b.windows = windows_.get();
@@ -1092,12 +1099,8 @@ void NufftPlan::execute_f64(int batch, const void* input, void* output, uint64_t
     l.batch = batch;
     l.output = out;
     StageScope scope(&timer_, kStageInterpolation, stream);
-    // Staged regions pay off for one vector and wide windows (measured: w 13
-    // 1.5x faster; w 10 even; batches of 16 slower, whose window weights the
-    // thread-per-point kernel reuses across vectors).
-    if (batch == 1 && kernel_.width >= 11 && interpolate_region64_supported(grid_)) {
-      interpolate_region64_execute(grid_, l, static_cast<const uint32_t*>(offsets_.get()), bins_, interp_parts(),
-                                   stream);
+    if (rows_order_ && interp_strips()) {
+      interp_strips_execute64(grid_, l, stream);
     } else {
       interpolate_execute64(grid_, l, stream);
     }
@@ -1268,16 +1271,24 @@ void NufftPlan::spread_to(int64_t active_batch, const void* strengths, void* gri
   check_cuda(cudaGetLastError(), "spread launch");
 }
 
+bool NufftPlan::interp_strips() const {
+  return interp_strips_chosen(dim_, precision_ != B200NUFFT_PRECISION_F32, kernel_.width, point_count_, fine_count_);
+}
+
+bool NufftPlan::interp_rows_order() const { return type_ == 2 && (dim_ == 3 || interp_strips()); }
+
 GridParams NufftPlan::rows_grid(uint64_t* bins) const {
-  // Bins of one cell along y and z and 8 cells along x: sorted by these
-  // keys, the points come in the order of their support starts' (z, y)
-  // rows and 8-cell x segments.
+  // The strips of the matrix-product interpolation, x cell by cell; or (the
+  // other 3D plans) bins of one cell along y and z and 8 cells along x: a
+  // warp's 32 points then gather from few grid rows.
+  int32_t shift[3] = {3, 0, 0};
+  if (interp_strips()) interp_strip_shifts(precision_ != B200NUFFT_PRECISION_F32, shift);
   GridParams rows = grid_;
   uint64_t stride = 1;
-  for (int a = 0; a < 3; ++a) {
-    const int shift = a == 0 ? std::min(3, ilog2(fine_[0])) : 0;
-    rows.axis[a].shift = shift;
-    rows.axis[a].bins = static_cast<uint32_t>((fine_[a] + (int64_t{1} << shift) - 1) >> shift);
+  for (int a = 0; a < dim_; ++a) {
+    shift[a] = std::min(shift[a], ilog2(fine_[a]));
+    rows.axis[a].shift = shift[a];
+    rows.axis[a].bins = static_cast<uint32_t>((fine_[a] + (int64_t{1} << shift[a]) - 1) >> shift[a]);
     rows.axis[a].stride = static_cast<uint32_t>(stride);
     stride *= rows.axis[a].bins;
   }
@@ -1291,6 +1302,9 @@ void NufftPlan::keep_rows_order(const uint32_t* order, int64_t count, cudaStream
   check_cuda(cudaMemcpyAsync(kept, order, static_cast<size_t>(count) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                              stream),
              "keep row order");
+  // 2D plans can be asked for the bin order inside a graph capture, where
+  // nothing can be allocated.
+  if (dim_ == 2) unsorted_.reserve(static_cast<size_t>(count) * 2 * scalar_bytes(), "coordinates in the caller's order");
 }
 
 SortBuffers NufftPlan::sort_buffers(int64_t count) {
@@ -1315,15 +1329,15 @@ void NufftPlan::finish_bin_order(cudaStream_t stream) {
   uint32_t* offsets = static_cast<uint32_t*>(offsets_.get());
   const uint32_t* rows = static_cast<const uint32_t*>(rows_perm_.get());
   if (precision_ == B200NUFFT_PRECISION_F32) {
-    float* coords = static_cast<float*>(unsorted_.reserve(static_cast<size_t>(count) * 3 * sizeof(float),
+    float* coords = static_cast<float*>(unsorted_.reserve(static_cast<size_t>(count) * dim_ * sizeof(float),
                                                            "coordinates in the caller's order"));
-    scatter_points3(static_cast<const float*>(sorted_points_.get()), rows, count, coords, stream);
+    scatter_points(static_cast<const float*>(sorted_points_.get()), rows, count, dim_, coords, stream);
     sort_points(coords, count, grid_, KeyKind::ApproximateCell, bins_, buf, offsets, &perm_, &sorted_keys_,
                 stream, &timer_);
   } else {
-    double* coords = static_cast<double*>(unsorted_.reserve(static_cast<size_t>(count) * 3 * sizeof(double),
+    double* coords = static_cast<double*>(unsorted_.reserve(static_cast<size_t>(count) * dim_ * sizeof(double),
                                                              "coordinates in the caller's order"));
-    scatter_points3(static_cast<const double*>(sorted_points_.get()), rows, count, coords, stream);
+    scatter_points(static_cast<const double*>(sorted_points_.get()), rows, count, dim_, coords, stream);
     sort_points64(coords, count, grid_, bins_, buf, offsets, &perm_, &sorted_keys_, stream, &timer_, nullptr);
   }
   check_cuda(cudaGetLastError(), "bin order launch");

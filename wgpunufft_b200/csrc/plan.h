@@ -150,23 +150,25 @@ class NufftPlan {
   DeviceBuffer part_cap_;    // type-1 plans: records per part, sized on the device
   DeviceBuffer windows_;  // f32 plans: PreparedWindow per slot
   DeviceBuffer inverse_;  // batched 2D f32 type-2 plans: slot of every point
-  // 2D type-2 plans: the bins' slots in parts of at most kInterpPartSlots
-  // (work items of the bin interpolation kernels).
+  // 2D f32 type-2 plans that interpolate by bins: the bins' slots in parts of
+  // at most kInterpPartSlots (work items of those kernels).
   DeviceBuffer interp_parts_, interp_part_start_, interp_part_bin_;
   int64_t interp_parts_bound_ = 0;
   void prepare_interp_parts(const uint32_t* offsets, cudaStream_t stream);
   InterpParts interp_parts() const;
   DeviceBuffer staged_;   // batched 2D f32 type-2 plans: values in slot order
-  // 3D type-2 plans: the interpolation's point order (support starts'
-  // (z, y) rows, 8-cell x segments), in which the sorted coordinates (and the
+  // 3D type-2 plans, and 2D ones that interpolate by strips: the
+  // interpolation's own point order, in which the sorted coordinates (and the
   // prepared windows of f32 plans) are kept; the reference's bin order stays
   // in perm_.
+  bool interp_strips() const;      // matrix products over strips (interp_strips.cu)
+  bool interp_rows_order() const;  // whether the plan keeps such an order
   bool rows_order_ = false;
   DeviceBuffer rows_perm_, rows_offsets_;
   const uint32_t* interp_perm() const {
     return rows_order_ ? static_cast<const uint32_t*>(rows_perm_.get()) : perm_;
   }
-  // The bins of that order (one cell along y and z, 8 along x) and their count.
+  // The bins of that order and their count.
   GridParams rows_grid(uint64_t* bins) const;
   // Copies a sort's permutation into rows_perm_ (the sort buffers are reused).
   void keep_rows_order(const uint32_t* order, int64_t count, cudaStream_t stream);

@@ -799,14 +799,19 @@ void sort_from_keys(int64_t count, uint64_t bins, int passes, SortBuffers buf, u
 }  // namespace
 
 template <typename T>
-void scatter_points3(const T* sorted, const uint32_t* perm, int64_t count, T* points, cudaStream_t stream) {
+void scatter_points(const T* sorted, const uint32_t* perm, int64_t count, int dimensions, T* points,
+                    cudaStream_t stream) {
   if (count == 0) return;
   const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
-  scatter_points_kernel<3, T><<<blocks, 256, 0, stream>>>(sorted, perm, count, points);
+  if (dimensions == 2) {
+    scatter_points_kernel<2, T><<<blocks, 256, 0, stream>>>(sorted, perm, count, points);
+  } else {
+    scatter_points_kernel<3, T><<<blocks, 256, 0, stream>>>(sorted, perm, count, points);
+  }
   note_launch();
 }
-template void scatter_points3<float>(const float*, const uint32_t*, int64_t, float*, cudaStream_t);
-template void scatter_points3<double>(const double*, const uint32_t*, int64_t, double*, cudaStream_t);
+template void scatter_points<float>(const float*, const uint32_t*, int64_t, int, float*, cudaStream_t);
+template void scatter_points<double>(const double*, const uint32_t*, int64_t, int, double*, cudaStream_t);
 
 void gather_sorted_points64(const double* points, const uint32_t* perm, int64_t count,
                             int dimensions, double* sorted, cudaStream_t stream,
