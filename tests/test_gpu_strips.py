@@ -78,6 +78,27 @@ def test_f32_3d_differs_from_f64_by_rounding(kind, eps, n_modes, count, spread, 
         assert rel(got, want) < F32_ROUNDING + 0.2 * eps
 
 
+@pytest.mark.parametrize("n_modes, count, spread, batch", [
+    ((32, 32), 7, "uniform", 1),             # below the density of the rows
+    ((64, 64), 100_000, "uniform", 1),       # whole tiles, rows longer than a chunk
+    ((75, 41), 9_001, "uniform", 3),         # ragged tiles, rows shorter than a chunk
+    ((50, 300), 200_003, "crowded", 1),      # parts of one tile, rows of thousands of points
+    ((33, 90), 20_003, "edges", 2),          # windows that wrap, a point out of reach
+])
+def test_f32_2d_rows_differ_from_f64_by_rounding(n_modes, count, spread, batch):
+    import wgpunufft_b200 as w
+
+    eps = 1e-6  # width 7
+    rng = np.random.default_rng(13)
+    points = points_of(rng, spread, count, [2 * n for n in n_modes])
+    inputs = values(rng, batch, count)
+    total = int(np.prod(n_modes))
+    plan, got = transform(w, 1, n_modes, eps, w.Precision.F32, batch, points, inputs, total)
+    _, want = transform(w, 1, n_modes, eps, w.Precision.F64, batch, points, inputs, total)
+    assert plan.kernel_width() == 7
+    assert rel(got, want) < (20 * eps if spread == "edges" else F32_ROUNDING + 0.2 * eps)
+
+
 @pytest.mark.parametrize("kind", [1, 2])
 @pytest.mark.parametrize("eps", [1e-4, 1e-8, 1e-9, 1e-12, 1e-14])  # widths 5, 9, 10, 13, 15
 @pytest.mark.parametrize("n_modes, count, spread", [
@@ -102,3 +123,20 @@ def test_f64_matches_direct_sums(kind, eps, n_modes, count, spread):
         want[reach] = native.direct_type2(points[reach], inputs[0], n_modes)[0]
     bound = max((20 if len(n_modes) == 2 else 32) * eps, 2e-13)  # 2e-13: rounding of the sums and the FFT
     assert rel(got[0], want) < bound
+
+
+def test_bin_offsets_across_long_empty_stretches():
+    """Two crowds a few cells wide: all other bins of the grid are empty."""
+    import torch
+
+    import wgpunufft_b200 as w
+    from tests.test_gpu_type12 import oracle_order
+
+    rng = np.random.default_rng(14)
+    points = np.concatenate([rng.normal(-1.0, 0.01, (70_001, 2)), rng.normal(2.0, 0.01, (80_002, 2))]).astype(np.float32)
+    plan = w.NufftPlan.type1_gpu(w.NufftConfig((300, 200), 1e-5))
+    plan.set_points_gpu(torch.from_numpy(points).cuda())
+    perm, offsets = plan.bin_order()
+    ref_perm, ref_offsets, *_ = oracle_order(points, plan.fine_grid_shape(), 1e-5, 1)
+    assert np.array_equal(perm.numpy(), ref_perm)
+    assert np.array_equal(offsets.numpy(), ref_offsets)

@@ -17,9 +17,11 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// The 19 bits a tf32 operand keeps, and the exact remainder.
+// v to the nearest value of the 19 bits a tf32 operand keeps, and the exact
+// remainder, whose sign is then independent of v's: what the products drop
+// (the remainder's own last bits, low times low) does not add up.
 __device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
-  hi = __float_as_uint(v) & 0xFFFFE000u;
+  hi = (__float_as_uint(v) + 0x1000u) & 0xFFFFE000u;
   lo = __float_as_uint(v - __uint_as_float(hi));
 }
 

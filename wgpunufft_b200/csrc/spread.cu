@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "device.h"
 #include "spread.h"
@@ -795,6 +796,31 @@ __device__ void spread_warp3_f64(const SpreadParams& sp, const double* points, c
   }
 }
 
+template <int D, int W, typename T>
+__host__ __device__ constexpr bool row_capable() {
+  return D == 2 && T::kPreparedWindows && W == kRowWidth;
+}
+
+// Shared memory of a CTA: the tile under the largest of its layouts, then the
+// record order and the staged records.
+template <int D, int W, typename T>
+__host__ __device__ inline size_t spread_tile_bytes(const SpreadParams& sp) {
+  int span = sp.padded_cells;
+  if (warp_capable<D, W, T>() && sp.span > span) span = sp.span;
+  if (strip_capable<D, W, T>() && sp.strip_pitch01 * sp.pad[2] > span) span = sp.strip_pitch01 * sp.pad[2];
+  return static_cast<size_t>(T::kWordsPerCell) * span * sizeof(typename T::Word);
+}
+template <int D, int W, typename T>
+__host__ __device__ constexpr size_t spread_aux_bytes() {
+  if (row_capable<D, W, T>()) return sizeof(float) * kSpreadWarps * kRowFloats;
+  const size_t order = sizeof(uint32_t) * (kWarpMaxRecords + 2 * kStripMax + 4);
+  if (strip_capable<D, W, T>()) {
+    return order + kSpreadWarps * (sizeof(typename T::Real) == 8 ? sizeof(double) * Strip64<W>::kDoubles
+                                                                 : sizeof(float) * kStripFloats);
+  }
+  return warp_capable<D, W, T>() ? order + sizeof(float) * kSpreadWarps * kWarpGroup * kStageStride : 0;
+}
+
 // Resident CTAs per SM that the register budget is sized for: three for narrow
 // windows without register runs, two for register runs, f64 windows, the 3D
 // warp spreader and the strips.
@@ -932,18 +958,23 @@ __device__ __forceinline__ void spread_part(
   // which leaves that much headroom in the scale.
   constexpr int kRun = spread_run<D, W, T>();
   constexpr bool kStripCapable = strip_capable<D, W, T>();
-  __shared__ uint32_t sorted[kWarpCapable || kStripCapable ? kWarpMaxRecords : 1];
-  __shared__ uint32_t strip_start[kStripCapable ? kStripMax + 1 : 1];
-  __shared__ uint32_t strip_cell[kStripCapable ? kStripMax : 1];
   constexpr bool kStrip64 = kStripCapable && sizeof(Real) == 8;
-  constexpr int kStageFloats = kStrip64 ? 2 * Strip64<W>::kDoubles
-                                        : (kStripCapable ? kStripFloats : (kWarpCapable ? kWarpGroup * kStageStride : 4));
-  __shared__ __align__(16) float stage[(kWarpCapable || kStripCapable ? kSpreadWarps : 1) * kStageFloats];
+  // 2D f32: bin rows whose windows reach at most 8 rows of cells take the products.
+  constexpr bool kRowCapable = row_capable<D, W, T>();
+  // The order and the staged records, after the tile (spread_aux_bytes).
+  uint32_t* const sorted = reinterpret_cast<uint32_t*>(shared_bytes + spread_tile_bytes<D, W, T>(sp));
+  uint32_t* const strip_start = sorted + (kRowCapable ? 0 : kWarpMaxRecords);
+  uint32_t* const strip_cell = strip_start + (kRowCapable ? 0 : kStripMax + 4);
+  float* const stage = reinterpret_cast<float*>(strip_cell + (kRowCapable ? 0 : kStripMax));
   const int tile_cells = sp.tile[0] * sp.tile[1] * sp.tile[2];
   const bool bucket = warp_path && record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
                       (tile_cells + 1) * kSpreadWarps <= T::kWordsPerCell * span &&
                       tile_total >= static_cast<uint32_t>(tile_cells);
-  int S = T::exponent(max_bits[b]) - (kRun > 1 ? kRunBits : 0);
+  const bool row_path = kRowCapable && sp.tile[0] <= kRowMaxTile && (1 << sp.grid.axis[1].shift) <= 9 - W &&
+                        2 * tile_total >= static_cast<uint32_t>(tile_cells);
+  // (A warp's register sums hold at most 2^11 records of magnitude below
+  // 2^27: below 2^38, which add_split takes.)
+  int S = T::exponent(max_bits[b]) - (row_path ? 3 : (kRun > 1 ? kRunBits : 0));
   const Real scale_lo = T::power_of_two(S / 2);
   const Real scale_hi = T::power_of_two(S - S / 2);
   const typename T::Complex* sv = strengths + static_cast<int64_t>(b) * point_count;
@@ -957,7 +988,8 @@ __device__ __forceinline__ void spread_part(
     constexpr int kS = 9 - W;
     const int strips = ((sp.tile[0] + kStripX - 1) / kStripX) * ((sp.tile[1] + kS - 1) / kS) *
                        ((sp.tile[2] + kS - 1) / kS);
-    strip_path = sp.strip_pitch0 > 0 && strips <= kStripMax && record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
+    strip_path = sp.strip_pitch0 > 0 && strips <= kStripMax &&
+                 record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
                  (strips * kStripX + 1) * kSpreadWarps <= T::kWordsPerCell * span &&
                  tile_total * static_cast<uint32_t>(strip_cells_per_record(W)) >= static_cast<uint32_t>(tile_cells);
     if (strip_path) {
@@ -1054,7 +1086,14 @@ __device__ __forceinline__ void spread_part(
         }
       }
     }
-  } else if constexpr (kRun > 1) {
+  }
+  if constexpr (kRowCapable) {
+    if (row_path) {
+      spread_rows2<W>(sp, static_cast<const PreparedWindow<2>*>(windows), sv, perm, row_begin, row_prefix, rows,
+                      origin, record_begin, record_end, acc, padded, stage, scale_lo, scale_hi);
+    }
+  }
+  if constexpr (kRun > 1) {
     // Each thread takes runs of up to kRun consecutive records (consecutive
     // slots of one bin row share starts when bins are one cell wide), sized so
     // that every pass gives every thread the same number of records.
@@ -1063,7 +1102,7 @@ __device__ __forceinline__ void spread_part(
     const uint32_t per_thread = (count + kSpreadThreads - 1) / kSpreadThreads;
     const uint32_t passes = (per_thread + kRun - 1) / kRun;
     const uint32_t run = passes ? (count + kSpreadThreads * passes - 1) / (kSpreadThreads * passes) : 1u;
-    for (uint32_t first = record_begin + tid * run; first < record_end; first += kSpreadThreads * run) {
+    for (uint32_t first = record_begin + tid * run; !row_path && first < record_end; first += kSpreadThreads * run) {
       const uint32_t stop = min(first + run, record_end);
       typename T::Complex a2[R][W];  // (re, im) register sums of the run
 #pragma unroll
@@ -1160,8 +1199,8 @@ __device__ __forceinline__ void spread_part(
   const float down_lo = T::kPreparedWindows ? ldexpf(1.0f, -S / 2) : 0.0f;
   const float down_hi = T::kPreparedWindows ? ldexpf(1.0f, -S - (-S / 2)) : 0.0f;
   auto value = [&](int which, int at) {
-    if constexpr (kStripCapable && !kStrip64) {
-      if (strip_path) {
+    if constexpr ((kStripCapable && !kStrip64) || kRowCapable) {
+      if (strip_path || row_path) {
         const float lo = static_cast<float>(static_cast<int32_t>(acc[(2 * which) * span + at]));
         const float hi = static_cast<float>(static_cast<int32_t>(acc[(2 * which + 1) * span + at]));
         return fmaf(hi, 65536.0f, lo) * down_lo * down_hi;
@@ -1551,9 +1590,7 @@ void fold_any(const SpreadParams& sp, int batch, const Complex* scratch, const u
 
 template <int D, int W, typename T>
 void launch_spread_width(const SpreadParams& sp, const SpreadLaunchT<T>& l, cudaStream_t stream) {
-  int span = warp_capable<D, W, T>() && sp.span > 0 ? sp.span : sp.padded_cells;
-  if (strip_capable<D, W, T>()) span = std::max(span, sp.strip_pitch01 * sp.pad[2]);
-  const size_t smem = static_cast<size_t>(T::kWordsPerCell) * span * sizeof(typename T::Word);
+  const size_t smem = spread_tile_bytes<D, W, T>(sp) + spread_aux_bytes<D, W, T>();
   auto kernel = spread_tiles_kernel<D, W, T>;
   check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)),
@@ -1781,10 +1818,20 @@ void spread_fold(const SpreadParams& sp, const SpreadLaunch& l, cudaStream_t str
 }
 
 size_t spread_shared_bytes(const SpreadParams& sp) {
-  const int w = sp.grid.width;
-  const bool warp = sp.grid.dimensions == 3 && w >= kWarpMinWidth && w <= kWarpMaxWidth && sp.span > 0;
-  const int span = std::max(warp ? sp.span : sp.padded_cells, sp.strip_pitch01 * sp.pad[2]);
-  return static_cast<size_t>(F32Traits::kWordsPerCell) * span * sizeof(uint32_t);
+  auto bytes = [&](auto width) {
+    constexpr int W = decltype(width)::value;
+    return sp.grid.dimensions == 2 ? spread_tile_bytes<2, W, F32Traits>(sp) + spread_aux_bytes<2, W, F32Traits>()
+                                   : spread_tile_bytes<3, W, F32Traits>(sp) + spread_aux_bytes<3, W, F32Traits>();
+  };
+  switch (sp.grid.width) {
+    case 2: return bytes(std::integral_constant<int, 2>());
+    case 3: return bytes(std::integral_constant<int, 3>());
+    case 4: return bytes(std::integral_constant<int, 4>());
+    case 5: return bytes(std::integral_constant<int, 5>());
+    case 6: return bytes(std::integral_constant<int, 6>());
+    case 7: return bytes(std::integral_constant<int, 7>());
+    default: return bytes(std::integral_constant<int, 8>());
+  }
 }
 
 void spread_count_parts(const SpreadParams& sp, const uint32_t* offsets, uint32_t* parts,

@@ -393,6 +393,193 @@ __device__ void spread_strips3(const SpreadParams& sp, const PreparedWindow<3>* 
   }
 }
 
+// 2D f32 tiles: the bin rows of a tile are strips already, in x order up to
+// the bins' width, as long as a row's windows reach at most 8 rows of cells
+// (bins of at most 9 - w cells along y), so no order is built. A warp takes an
+// equal range of consecutive records; for 8 points of one bin row,
+//   C[(y, re/im), x] += sum_k (c wy)[(y, re/im), k] wx[k, x]
+// is one 16 x 8 x 8 product per block of 8 columns that their windows reach,
+// in split tf32 as for the 3D strips. A row's blocks reach the tile when the
+// range leaves the row.
+constexpr int kRowBlocks = 9;      // blocks of 8 columns: 64 starts and the window
+constexpr int kRowMaxTile = 64;    // starts of a tile along x, at most
+// The width that takes them, where a tile holds a record per two start cells:
+// below w 7 the register runs of the per-point spreader are at least as fast
+// (1024^2 modes, 2 points per cell, w 6: 294 us against 408; w 7: 527 against
+// 492, crowded points 190 against 126; at 1/4 point per cell 185 against 197).
+constexpr int kRowWidth = 7;
+// Staged floats of a point: wx[8] wy[8] re im - -.
+constexpr int kRowStride = 20;
+constexpr int kRowFloats = 32 * kRowStride;
+
+template <int W>
+__device__ void spread_rows2(const SpreadParams& sp, const PreparedWindow<2>* win2, const float2* sv,
+                             const uint32_t* perm, const uint32_t* row_begin, const uint32_t* row_prefix, int rows,
+                             const int* origin, uint32_t record_begin, uint32_t record_end, uint32_t* acc, int padded,
+                             float* stage, float scale_lo, float scale_hi) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  float* const st = stage + warp * kRowFloats;
+  const uint32_t n = record_end - record_begin;
+  const uint32_t share = (n + kSpreadWarps - 1) / kSpreadWarps;
+  uint32_t at = record_begin + min(n, share * warp);
+  const uint32_t to = record_begin + min(n, share * (warp + 1));
+  if (at >= to) return;
+  const int bin_first = origin[1] >> sp.grid.axis[1].shift;  // the tile's first bin row
+  int row = 0;
+  {
+    int low = 0, high = rows - 1;  // last row starting at or before `at`
+    while (low < high) {
+      const int mid = (low + high + 1) >> 1;
+      if (row_prefix[mid] <= at) low = mid; else high = mid - 1;
+    }
+    row = low;
+  }
+  float2 sum[kRowBlocks][2];  // columns 8 j + 2 t, + 1 of row g: real and imaginary parts
+#pragma unroll
+  for (int j = 0; j < kRowBlocks; ++j) sum[j][0] = sum[j][1] = make_float2(0.0f, 0.0f);
+  int col_lo = kRowBlocks, col_hi = -1;
+  // Lane = point of the chunk (up to 32 records of one row). The next chunk's
+  // windows and point indexes are loaded one chunk ahead.
+  struct Rows {
+    int row;
+    uint32_t at, end;
+  };
+  auto settle = [&](Rows& r) {  // the row holding record r.at
+    while (r.row + 1 < rows && r.at >= row_prefix[r.row + 1]) ++r.row;
+    r.end = min(min(r.at + 32u, row_prefix[r.row + 1]), to);
+  };
+  auto fetch = [&](const Rows& r, int4& win, uint32_t& point) {
+    win.x = -1;
+    if (r.at < to && r.at + lane < r.end) {
+      const uint32_t slot = row_begin[r.row] + (r.at + lane - row_prefix[r.row]);
+      win = __ldg(reinterpret_cast<const int4*>(win2 + slot));
+      point = __ldg(perm + slot);
+    }
+  };
+  Rows now{row, at, at};
+  settle(now);
+  int4 win0, win1;
+  uint32_t q0 = 0, q1 = 0;
+  fetch(now, win0, q0);
+  float2 c0 = make_float2(0.0f, 0.0f);
+  if (win0.x >= 0) c0 = __ldg(sv + q0);
+  for (;;) {
+    Rows next{now.row, now.end, now.end};
+    if (next.at < to) settle(next);
+    fetch(next, win1, q1);
+    // Stage the chunk. Points outside the fold's reach or starting in another
+    // tile weigh zero.
+    const int y_first = max((bin_first + now.row) << sp.grid.axis[1].shift, origin[1]);  // first start of the row
+    const int x = win0.x - origin[0], y = win0.y - origin[1];
+    const bool inside = win0.x >= 0 && x >= 0 && x < sp.tile[0] && y >= 0 && y < sp.tile[1];
+    float wx[W], wy[W];
+    horner32_window<W>(__int_as_float(win0.z), sp.grid.horner32, wx);
+    horner32_window<W>(__int_as_float(win0.w), sp.grid.horner32, wy);
+    __syncwarp();  // the previous chunk's rows are read
+    {
+      float* const mine = st + lane * kRowStride;
+      float row_x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) row_x[j] = j < W ? wx[j] : 0.0f;
+      float4* const mine4 = reinterpret_cast<float4*>(mine);
+      mine4[0] = make_float4(row_x[0], row_x[1], row_x[2], row_x[3]);
+      mine4[1] = make_float4(row_x[4], row_x[5], row_x[6], row_x[7]);
+      mine4[2] = mine4[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const int place = inside ? win0.y - y_first : 0;
+#pragma unroll
+      for (int j = 0; j < W; ++j) mine[8 + place + j] = wy[j];
+      const float2 c = inside ? cscale(cscale(c0, scale_lo), scale_hi) : make_float2(0.0f, 0.0f);
+      *reinterpret_cast<float2*>(mine + 16) = c;
+    }
+    __syncwarp();
+    const int count = static_cast<int>(now.end - now.at);
+    float2 c1 = make_float2(0.0f, 0.0f);
+    if (win1.x >= 0) c1 = __ldg(sv + q1);
+#pragma unroll 1
+    for (int k = 0; k < count; k += 8) {
+      // Columns of the eight points' windows.
+      const bool member = inside && (lane >> 3) == (k >> 3);
+      const int lo = __reduce_min_sync(0xFFFFFFFFu, member ? x : 0x7FFF) >> 3;
+      const int hi = (__reduce_max_sync(0xFFFFFFFFu, member ? x : -W) + W - 1) >> 3;
+      const int x0 = g - __shfl_sync(0xFFFFFFFFu, x, k + t), x1 = g - __shfl_sync(0xFFFFFFFFu, x, k + 4 + t);
+      const float* const p0 = st + (k + t) * kRowStride;
+      const float* const p1 = p0 + 4 * kRowStride;
+      uint32_t ah[4], al[4];
+      {
+        const float y0 = p0[8 + g], y1 = p1[8 + g];
+        const float2 v0 = *reinterpret_cast<const float2*>(p0 + 16);
+        const float2 v1 = *reinterpret_cast<const float2*>(p1 + 16);
+        split_tf32(v0.x * y0, ah[0], al[0]);
+        split_tf32(v0.y * y0, ah[1], al[1]);
+        split_tf32(v1.x * y1, ah[2], al[2]);
+        split_tf32(v1.y * y1, ah[3], al[3]);
+      }
+      col_lo = min(col_lo, lo);
+      col_hi = max(col_hi, hi);
+      auto block = [&](int j) {  // j: a constant of the caller
+        const unsigned i0 = static_cast<unsigned>(x0 + 8 * j), i1 = static_cast<unsigned>(x1 + 8 * j);
+        uint32_t bh0, bl0, bh1, bl1;
+        split_tf32(i0 < 8u ? p0[i0] : 0.0f, bh0, bl0);
+        split_tf32(i1 < 8u ? p1[i1] : 0.0f, bh1, bl1);
+        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_tf32(d, ah, bl0, bl1);
+        mma_tf32(d, al, bh0, bh1);
+        mma_tf32(d, ah, bh0, bh1);
+        sum[j][0] = __fadd2_rn(sum[j][0], make_float2(d[0], d[1]));
+        sum[j][1] = __fadd2_rn(sum[j][1], make_float2(d[2], d[3]));
+      };
+      // Blocks lo .. hi: a jump to the first, and on while there are more.
+      switch (lo) {
+#define B200NUFFT_ROW_BLOCK(J) \
+  case J:                      \
+    block(J);                  \
+    if (hi <= J) break;        \
+    [[fallthrough]];
+        B200NUFFT_ROW_BLOCK(0)
+        B200NUFFT_ROW_BLOCK(1)
+        B200NUFFT_ROW_BLOCK(2)
+        B200NUFFT_ROW_BLOCK(3)
+        B200NUFFT_ROW_BLOCK(4)
+        B200NUFFT_ROW_BLOCK(5)
+        B200NUFFT_ROW_BLOCK(6)
+        B200NUFFT_ROW_BLOCK(7)
+#undef B200NUFFT_ROW_BLOCK
+        case 8: block(8); break;
+        default: break;  // no point of these in the tile
+      }
+    }
+    const bool done = next.at >= to;
+    if (done || next.row != now.row) {
+      const int cy = y_first - origin[1] + g;
+      constexpr float kMagic = 12582912.0f;  // 1.5 x 2^23
+      const float2 magic = make_float2(kMagic, kMagic), minus = make_float2(-kMagic, -kMagic);
+      const float2 down = make_float2(1.0f / 65536.0f, 1.0f / 65536.0f), up = make_float2(-65536.0f, -65536.0f);
+#pragma unroll
+      for (int j = 0; j < kRowBlocks; ++j) {
+        if (j >= col_lo && j <= col_hi) {
+          const int cx = 8 * j + 2 * t, cell = cy * sp.pad[0] + cx;
+          const bool in0 = cy < sp.pad[1] && cx < sp.pad[0], in1 = cy < sp.pad[1] && cx + 1 < sp.pad[0];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float2 h = __ffma2_rn(sum[j][i], down, magic);
+            const float2 l = __fadd2_rn(__ffma2_rn(__fadd2_rn(h, minus), up, sum[j][i]), magic);
+            if (in0) add_split(acc, padded, i, cell, h.x, l.x);
+            if (in1) add_split(acc, padded, i, cell + 1, h.y, l.y);
+            sum[j][i] = make_float2(0.0f, 0.0f);
+          }
+        }
+      }
+      col_lo = kRowBlocks;
+      col_hi = -1;
+    }
+    if (done) return;
+    now = next;
+    win0 = win1;
+    c0 = c1;
+  }
+}
+
 // 2D f64 tiles: strips of 16 x S cells (x, y) reach YT x NT blocks of 8 x 8
 // cells, and 4 points add
 //   C[y, x] += sum_k (c wy)[y, k] wx[k, x]
