@@ -106,6 +106,8 @@ def test_f32_2d_rows_differ_from_f64_by_rounding(n_modes, count, spread, batch):
     ((40, 30), 20_003, "crowded"),
     ((9, 70), 6_001, "edges"),
     ((12, 14, 10), 20_001, "uniform"),
+    ((30, 8, 9), 6_003, "edges"),
+    ((15, 16, 17), 30_001, "crowded"),   # several parts of one tile
 ])
 def test_f64_matches_direct_sums(kind, eps, n_modes, count, spread):
     import wgpunufft_b200 as w

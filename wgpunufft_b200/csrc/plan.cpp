@@ -423,6 +423,14 @@ void NufftPlan::configure_tiles() {
     for (int a = 0; a < dim_; ++a) tile[a] = tuning.tile;
   }
   for (int a = 0; a < dim_; ++a) tile[a] = std::min(tile[a], pow2_ceil(fine_[a]));
+  // 3D f64 tiles spread in registers have the one shape that fills them.
+  const bool regs64 = dim_ == 3 && precision_ != B200NUFFT_PRECISION_F32 && w >= kReg64MinWidth && w <= kReg64MaxWidth;
+  if (regs64) {
+    tile[0] = kReg64Planes - w + 1;
+    tile[1] = 8 * reg64_blocks_y(w) - w + 1;
+    tile[2] = 8 * reg64_blocks_z(w) - w + 1;
+  }
+  sp.regs64 = regs64 ? 1 : 0;
   // The tensor-core spreader needs one-cell bin rows, column bins of at most
   // 8 cells, and its own tile shape (16 cells x 22 - w rows).
   tc_active_ = tc_enabled_ && grid_.axis[1].shift == 0 && grid_.axis[0].shift <= 3;
@@ -435,7 +443,7 @@ void NufftPlan::configure_tiles() {
     for (int a = 0; a < dim_; ++a) cells *= tile[a] + w - 1;
     return cells * 16;
   };
-  while (!tc_active_ && padded_bytes() > kTileBytesTarget) {
+  while (!tc_active_ && !regs64 && padded_bytes() > kTileBytesTarget) {
     int largest = dim_ - 1;
     for (int a = dim_ - 1; a >= 0; --a) {
       if (tile[a] > tile[largest]) largest = a;
@@ -454,8 +462,10 @@ void NufftPlan::configure_tiles() {
     sp.tile_count *= sp.ntiles[a];
     sp.padded_cells *= sp.pad[a];
     const int64_t side = int64_t(1) << grid_.axis[a].shift;
-    if (side > tile[a]) tiles_per_bin *= side / tile[a];
-    if (a > 0) rows *= std::max<int64_t>(1, tile[a] / side);
+    // Tiles that a bin can meet, and bins that a tile can: tiles of no whole
+    // number of bins (or bins of no whole number of tiles) share some.
+    if (tile[a] % side != 0) tiles_per_bin *= side % tile[a] == 0 ? side / tile[a] : (side + tile[a] - 2) / tile[a] + 1;
+    if (a > 0) rows *= tile[a] % side == 0 ? tile[a] / side : (side % tile[a] == 0 ? 1 : (tile[a] + side - 2) / side + 1);
   }
   for (int a = dim_; a < 3; ++a) {
     sp.tile[a] = 1;

@@ -53,6 +53,8 @@ struct SpreadParams {
   // padded tile under the tensor-core strips (spread_strip_layout).
   int32_t strip_pitch0;
   int32_t strip_pitch01;
+  // 3D f64 plans of widths kReg64MinWidth..kReg64MaxWidth: the tiles of spread_regs64.
+  int32_t regs64;
   // 3D plans of 16 x 16 x (4 k)-cell tiles whose cells' candidate lists are,
   // along every axis, ordered parts of the list of their tile's first cell
   // (checked on the host): single vectors fold per destination tile
@@ -101,6 +103,15 @@ constexpr int kStripMaxRecords = 2048;  // records of a part under the strips, a
 // Pitches of the padded tile (pad[a] cells, some slack allowed) that spread
 // a strip's flush, 8 rows x 4 even planes per warp, over the most banks.
 void spread_strip_layout(const int32_t pad[3], int32_t& pitch0, int32_t& pitch01);
+
+// 3D f64 plans of these widths spread in registers (spread_regs.cu): padded
+// tiles of kReg64Planes x 8 by x 8 bz cells, tiles of w - 1 fewer starts per
+// axis. Wider windows would leave tiles of three starts or less along z.
+constexpr int kReg64MinWidth = 5;
+constexpr int kReg64MaxWidth = 13;
+constexpr int kReg64Planes = 24;
+__host__ __device__ constexpr int reg64_blocks_y(int w) { return w <= 9 ? 2 : 3; }
+__host__ __device__ constexpr int reg64_blocks_z(int) { return 2; }
 
 struct SpreadLaunch {
   const float* points;    // coordinates in bin (slot) order
@@ -186,6 +197,8 @@ void exclusive_scan_u32(const uint32_t* in, int64_t n, uint32_t* out, cudaStream
 // Spreads `batch` strength vectors onto `fine`, overwriting every cell.
 void spread_execute(const SpreadParams& sp, const SpreadLaunch& launch, cudaStream_t stream,
                     StageTimer* timer = nullptr);
+// 3D f64 tiles in registers (SpreadParams::regs64), to the padded tiles.
+void spread_regs64(const SpreadParams& sp, const SpreadLaunch64& launch, cudaStream_t stream);
 void spread_execute64(const SpreadParams& sp, const SpreadLaunch64& launch, cudaStream_t stream,
                       StageTimer* timer = nullptr);
 
