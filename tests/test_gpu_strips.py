@@ -142,3 +142,31 @@ def test_bin_offsets_across_long_empty_stretches():
     ref_perm, ref_offsets, *_ = oracle_order(points, plan.fine_grid_shape(), 1e-5, 1)
     assert np.array_equal(perm.numpy(), ref_perm)
     assert np.array_equal(offsets.numpy(), ref_offsets)
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-2, 1e-3, 1e-4, 1e-5, 1e-6])  # widths 2 to 7
+@pytest.mark.parametrize("batch", [1, 3, 18])
+@pytest.mark.parametrize("n_modes, spread", [((40, 30), "crowded"), ((9, 70), "edges"), ((300, 200), "uniform")])
+def test_batched_2d_type2_strips_match_the_gather(eps, batch, n_modes, spread):
+    """The strips, asked for by the tensor-core method, against the CUDA-core
+    kernels on the same windows: rounding of both (F32_ROUNDING) apart."""
+    import torch
+
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(15)
+    count = 5_003
+    points = torch.from_numpy(points_of(rng, spread, count, [2 * n for n in n_modes])).cuda()
+    inputs = torch.from_numpy(values(rng, batch, int(np.prod(n_modes)))).cuda()
+
+    def run(method):
+        plan = w.NufftPlan.type2_gpu(w.NufftConfig(n_modes, eps, batch=batch, spread_method=method))
+        out = torch.empty((batch, count), dtype=torch.complex64, device="cuda")
+        plan.encode_type2_gpu(points, inputs, out)
+        first = out.clone()
+        plan.execute_type2_gpu(inputs, out)
+        plan.synchronize()
+        assert torch.equal(first.view(torch.int32), out.view(torch.int32))
+        return out.cpu().numpy()
+
+    assert rel(run(w.SpreadMethod.TENSOR_CORES), run(w.SpreadMethod.CUDA_CORES)) < F32_ROUNDING

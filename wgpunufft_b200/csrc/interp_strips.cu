@@ -28,6 +28,9 @@ namespace b200nufft {
 namespace {
 
 constexpr int kSpan = 16;  // x starts of a group, at most
+// Vectors of a CTA: each stages its points' weights once for them, and the
+// outputs that the running CTAs scatter to stay in L2 (4 x 2e6 points: 64 MB).
+constexpr int kBlockVectors = 4;
 
 // Strip sides (log2) along y and z: the rows a strip's windows reach fill the
 // contracted index (8 rows in f32, multiples of 4 in f64); z strips of 4.
@@ -62,7 +65,7 @@ struct F64Strips {
   static constexpr int kWarps = 2;
 };
 
-template <int D, int W, typename T>
+template <int D, int W, int V, typename T>
 __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
     GridParams grid, const typename T::Real* __restrict__ points, const void* __restrict__ windows, int64_t count,
     const uint32_t* __restrict__ perm, const typename T::Complex* __restrict__ fine, int batch,
@@ -159,10 +162,11 @@ __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
       }
     }
   }
+  const int first_vector = blockIdx.y * kBlockVectors, last_vector = min(first_vector + kBlockVectors, batch);
   if (exists && !reach) {
     Complex zero;
     zero.x = zero.y = Real(0);
-    for (int b = 0; b < batch; ++b) output[static_cast<int64_t>(b) * count + point] = zero;
+    for (int b = first_vector; b < last_vector; ++b) output[static_cast<int64_t>(b) * count + point] = zero;
   }
   __syncwarp();
 
@@ -219,11 +223,21 @@ __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
       while (y >= n1) y -= n1;
       row_at[k] = static_cast<int64_t>(y) * n0;
     }
-    for (int b = 0; b < batch; ++b) {
-      const Real* const values = reinterpret_cast<const Real*>(fine + static_cast<int64_t>(b) * grid.fine_count) + (g & 1);
-      Complex v[4];
+    // V vectors at a time share the weights; the last pass of a batch that V
+    // does not divide repeats its last vector.
+    for (int b = first_vector; b < last_vector; b += V) {
+      const Real* values[V];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) v[m].x = v[m].y = Real(0);
+      for (int k = 0; k < V; ++k) {
+        const int vector = min(b + k, last_vector - 1);
+        values[k] = reinterpret_cast<const Real*>(fine + static_cast<int64_t>(vector) * grid.fine_count) + (g & 1);
+      }
+      Complex v[V][4];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) v[k][m].x = v[k][m].y = Real(0);
+      }
       for (int n = lx >> 2; n <= hx >> 2; ++n) {
         int column = 4 * n + (g >> 1);
         column = column >= n0 ? column - n0 : column;
@@ -237,51 +251,63 @@ __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
 #pragma unroll 2
         for (int z = z_lo; z <= z_hi; ++z) {
           const int64_t plane = D == 3 ? static_cast<int64_t>(z >= n2 ? z - n2 : z) * plane_cells : 0;
-          const Real* const at = values + 2 * (plane + column);
           Real weight[4];
 #pragma unroll
           for (int m = 0; m < 4; ++m) {
             weight[m] = wx[m];
             if (D == 3) weight[m] *= weights_z[8 * m * S::kPitchZ + z];
           }
-          if constexpr (!F64) {
-            uint32_t bh0, bl0, bh1, bl1;
-            split_tf32(__ldg(at + 2 * row_at[0]), bh0, bl0);
-            split_tf32(__ldg(at + 2 * row_at[1]), bh1, bl1);
 #pragma unroll
-            for (int m = 0; m < 2; ++m) {
-              float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-              mma_tf32(d, al[m], bh0, bh1);
-              mma_tf32(d, ah[m], bl0, bl1);
-              mma_tf32(d, ah[m], bh0, bh1);
-              v[2 * m] = cfma(make_float2(d[0], d[1]), weight[2 * m], v[2 * m]);
-              v[2 * m + 1] = cfma(make_float2(d[2], d[3]), weight[2 * m + 1], v[2 * m + 1]);
+          for (int k = 0; k < V; ++k) {
+            const Real* const at = values[k] + 2 * (plane + column);
+            if constexpr (!F64) {
+              uint32_t bh0, bl0, bh1, bl1;
+              split_tf32(__ldg(at + 2 * row_at[0]), bh0, bl0);
+              split_tf32(__ldg(at + 2 * row_at[1]), bh1, bl1);
+#pragma unroll
+              for (int m = 0; m < 2; ++m) {
+                float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma_tf32(d, al[m], bh0, bh1);
+                mma_tf32(d, ah[m], bl0, bl1);
+                mma_tf32(d, ah[m], bh0, bh1);
+                v[k][2 * m] = cfma(make_float2(d[0], d[1]), weight[2 * m], v[k][2 * m]);
+                v[k][2 * m + 1] = cfma(make_float2(d[2], d[3]), weight[2 * m + 1], v[k][2 * m + 1]);
+              }
+            } else {
+              double2 d[4];
+#pragma unroll
+              for (int m = 0; m < 4; ++m) d[m] = make_double2(0.0, 0.0);
+#pragma unroll
+              for (int i = 0; i < K; ++i) {
+                const double value = __ldg(at + 2 * row_at[i]);
+#pragma unroll
+                for (int m = 0; m < 4; ++m) mma_f64(d[m], a64[m][i], value);
+              }
+#pragma unroll
+              for (int m = 0; m < 4; ++m) v[k][m] = cfma(d[m], weight[m], v[k][m]);
             }
-          } else {
-            double2 d[4];
-#pragma unroll
-            for (int m = 0; m < 4; ++m) d[m] = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-              const double value = __ldg(at + 2 * row_at[k]);
-#pragma unroll
-              for (int m = 0; m < 4; ++m) mma_f64(d[m], a64[m][k], value);
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) v[m] = cfma(d[m], weight[m], v[m]);
           }
         }
       }
-      // The columns' sums; lane t keeps point 8 t + g.
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        v[m].x += __shfl_xor_sync(0xFFFFFFFFu, v[m].x, 1);
-        v[m].y += __shfl_xor_sync(0xFFFFFFFFu, v[m].y, 1);
-        v[m].x += __shfl_xor_sync(0xFFFFFFFFu, v[m].x, 2);
-        v[m].y += __shfl_xor_sync(0xFFFFFFFFu, v[m].y, 2);
+      for (int k = 0; k < V; ++k) {
+        // The columns' sums, halved twice: lane t ends with point 8 t + g.
+        const bool upper = (t & 2) != 0, odd = (t & 1) != 0;
+        Complex half[2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const Complex keep = upper ? v[k][2 + m] : v[k][m], give = upper ? v[k][m] : v[k][2 + m];
+          half[m].x = keep.x + __shfl_xor_sync(0xFFFFFFFFu, give.x, 2);
+          half[m].y = keep.y + __shfl_xor_sync(0xFFFFFFFFu, give.y, 2);
+        }
+        const Complex keep = odd ? half[1] : half[0], give = odd ? half[0] : half[1];
+        Complex e;
+        e.x = keep.x + __shfl_xor_sync(0xFFFFFFFFu, give.x, 1);
+        e.y = keep.y + __shfl_xor_sync(0xFFFFFFFFu, give.y, 1);
+        if (((members >> (8 * t + g)) & 1u) && b + k < last_vector) {
+          output[static_cast<int64_t>(b + k) * count + destination] = e;
+        }
       }
-      const Complex e = t == 0 ? v[0] : (t == 1 ? v[1] : (t == 2 ? v[2] : v[3]));
-      if ((members >> (8 * t + g)) & 1u) output[static_cast<int64_t>(b) * count + destination] = e;
     }
   }
 }
@@ -290,9 +316,18 @@ template <int D, int W, typename T>
 void launch_width(const GridParams& g, const typename T::Real* points, const void* windows, int64_t count,
                   const uint32_t* perm, const typename T::Complex* fine, int batch, typename T::Complex* output,
                   cudaStream_t stream) {
-  const unsigned blocks = static_cast<unsigned>((count + 32 * T::kWarps - 1) / (32 * T::kWarps));
-  interp_strips_kernel<D, W, T><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count, perm, fine, batch,
-                                                                       output);
+  const dim3 blocks(static_cast<unsigned>((count + 32 * T::kWarps - 1) / (32 * T::kWarps)),
+                    static_cast<unsigned>((batch + kBlockVectors - 1) / kBlockVectors));
+  if constexpr (D == 2 && sizeof(typename T::Real) == 4) {
+    if (batch > 1) {
+      interp_strips_kernel<D, W, kBlockVectors, T><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count,
+                                                                                          perm, fine, batch, output);
+      note_launch();
+      return;
+    }
+  }
+  interp_strips_kernel<D, W, 1, T><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count, perm, fine, batch,
+                                                                          output);
   note_launch();
 }
 
@@ -317,6 +352,17 @@ void interp_strips_execute(const GridParams& g, const InterpLaunch& l, cudaStrea
   auto launch = [&](auto kernel) {
     kernel(g, l.points, l.windows, l.point_count, l.perm, l.fine, l.batch, l.output, stream);
   };
+  if (g.dimensions == 2) {
+    switch (g.width) {
+      case 2: launch(launch_width<2, 2, F32Strips>); break;
+      case 3: launch(launch_width<2, 3, F32Strips>); break;
+      case 4: launch(launch_width<2, 4, F32Strips>); break;
+      case 5: launch(launch_width<2, 5, F32Strips>); break;
+      case 6: launch(launch_width<2, 6, F32Strips>); break;
+      default: launch(launch_width<2, 7, F32Strips>); break;
+    }
+    return;
+  }
   switch (g.width) {
     case 6: launch(launch_width<3, 6, F32Strips>); break;
     default: launch(launch_width<3, 7, F32Strips>); break;

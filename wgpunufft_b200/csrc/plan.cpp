@@ -687,7 +687,8 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
                                      : nullptr;
   const size_t sorted_bytes = static_cast<size_t>(std::max<int64_t>(count, 1)) * dim_ * scalar_bytes();
   if (precision_ == B200NUFFT_PRECISION_F32) {
-    tc2_active_ = tc2_enabled_ && tc_interp_supported(grid_);
+    tc2_active_ = tc2_enabled_ && batch_ >= kTi2Vectors && tc_interp_supported(grid_);
+    tc2_strips_ = tc2_enabled_ && !tc2_active_;
     if (tc2_active_ && count > 0) {
       // The tensor-core order first (its permutation is consumed at once),
       // then the reference's type-2 bins in the same sort buffers.
@@ -722,6 +723,29 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       tc_interp_prepare(tc2_grid_, p, stream);
       tc2_part_upper_bound_ = tiles + chunk_bound / kTi2ChunksPerPart + 1;
       tc2_vector_max_.reserve(static_cast<size_t>(std::max<int64_t>(batch_, 1)) * sizeof(uint32_t), "vector maxima");
+    }
+    if (tc2_strips_ && count > 0) {
+      // The strip order and its windows first (the sort buffers then take the
+      // reference's type-2 bins).
+      uint64_t bins2 = 0;
+      const GridParams strips = strips_grid(&bins2);
+      uint32_t* offsets2 =
+          static_cast<uint32_t*>(tc2_offsets_.reserve((bins2 + 1) * sizeof(uint32_t), "strip offsets"));
+      uint32_t* order = nullptr;
+      uint32_t* keys2 = nullptr;
+      sort_points(static_cast<const float*>(points), count, strips, KeyKind::SupportStart, bins2, buf, offsets2,
+                  &order, &keys2, stream, &timer_);
+      uint32_t* kept = static_cast<uint32_t*>(
+          tc2_perm_.reserve(static_cast<size_t>(count) * sizeof(uint32_t), "strip permutation"));
+      check_cuda(cudaMemcpyAsync(kept, order, static_cast<size_t>(count) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                                 stream),
+                 "keep strip order");
+      float* sorted = static_cast<float*>(sorted_points_.reserve(sorted_bytes, "sorted coordinates"));
+      gather_sorted_points(static_cast<const float*>(points), kept, count, dim_, sorted, stream, &timer_);
+      StageScope scope(&timer_, kStageBinOffsets, stream);
+      prepare_windows(sorted, count, grid_,
+                      tc2_windows_.reserve(static_cast<size_t>(count) * prepared_window_bytes(dim_), "strip windows"),
+                      stream);
     }
     // The interpolation's own order (rows_grid) is sorted here and its
     // permutation kept; the reference's bins are sorted when they are asked for.
@@ -989,6 +1013,19 @@ void NufftPlan::execute_f32(int batch, const void* input, void* output, uint64_t
       t.error_flag = static_cast<uint32_t*>(counters_.get()) + 7;
       StageScope scope(&timer_, kStageInterpolation, stream);
       tc_interp_execute(tc2_grid_, t, stream);
+      return;
+    }
+    if (tc2_strips_ && strips_for_batch(batch)) {
+      InterpLaunch l;
+      l.points = nullptr;
+      l.windows = tc2_windows_.get();
+      l.point_count = point_count_;
+      l.perm = static_cast<const uint32_t*>(tc2_perm_.get());
+      l.fine = fine;
+      l.batch = batch;
+      l.output = static_cast<float2*>(output);
+      StageScope scope(&timer_, kStageInterpolation, stream);
+      interp_strips_execute(grid_, l, stream);
       return;
     }
     if (rows_order_ && interp_strips()) {
@@ -1285,25 +1322,43 @@ bool NufftPlan::interp_strips() const {
   return interp_strips_chosen(dim_, precision_ != B200NUFFT_PRECISION_F32, kernel_.width, point_count_, fine_count_);
 }
 
+bool NufftPlan::strips_for_batch(int batch) const {
+  // 2D 512^2 modes, 2e6 points, us per execution, per-bin regions of 32 vectors
+  // against strips: w 7, 16 vectors 1682 / 692, 32 vectors 1893 / 1369; w 4, 16
+  // vectors 919 / 648, 32 vectors 1056 / 1279. The tcgen05 kernel serves 64
+  // vectors for the price of 16 (w 7, 64 vectors: 2484 against 2727).
+  if (tc_min_batch_ == 1) return true;
+  return batch >= tc_min_batch_ && kernel_.width >= 3 && (kernel_.width >= 6 || batch <= 24);
+}
+
 bool NufftPlan::interp_rows_order() const { return type_ == 2 && (dim_ == 3 || interp_strips()); }
 
-GridParams NufftPlan::rows_grid(uint64_t* bins) const {
-  // The strips of the matrix-product interpolation, x cell by cell; or (the
-  // other 3D plans) bins of one cell along y and z and 8 cells along x: a
-  // warp's 32 points then gather from few grid rows.
-  int32_t shift[3] = {3, 0, 0};
-  if (interp_strips()) interp_strip_shifts(precision_ != B200NUFFT_PRECISION_F32, shift);
+GridParams NufftPlan::bins_grid(const int32_t sides_log2[3], uint64_t* bins) const {
   GridParams rows = grid_;
   uint64_t stride = 1;
   for (int a = 0; a < dim_; ++a) {
-    shift[a] = std::min(shift[a], ilog2(fine_[a]));
-    rows.axis[a].shift = shift[a];
-    rows.axis[a].bins = static_cast<uint32_t>((fine_[a] + (int64_t{1} << shift[a]) - 1) >> shift[a]);
+    rows.axis[a].shift = std::min(sides_log2[a], ilog2(fine_[a]));
+    rows.axis[a].bins = static_cast<uint32_t>((fine_[a] + (int64_t{1} << rows.axis[a].shift) - 1) >> rows.axis[a].shift);
     rows.axis[a].stride = static_cast<uint32_t>(stride);
     stride *= rows.axis[a].bins;
   }
   *bins = stride;
   return rows;
+}
+
+GridParams NufftPlan::strips_grid(uint64_t* bins) const {
+  int32_t shift[3];
+  interp_strip_shifts(precision_ != B200NUFFT_PRECISION_F32, shift);
+  return bins_grid(shift, bins);
+}
+
+GridParams NufftPlan::rows_grid(uint64_t* bins) const {
+  // The strips of the matrix-product interpolation, x cell by cell; or (the
+  // other 3D plans) bins of one cell along y and z and 8 cells along x: a
+  // warp's 32 points then gather from few grid rows.
+  if (interp_strips()) return strips_grid(bins);
+  const int32_t shift[3] = {3, 0, 0};
+  return bins_grid(shift, bins);
 }
 
 void NufftPlan::keep_rows_order(const uint32_t* order, int64_t count, cudaStream_t stream) {

@@ -168,7 +168,9 @@ class NufftPlan {
   const uint32_t* interp_perm() const {
     return rows_order_ ? static_cast<const uint32_t*>(rows_perm_.get()) : perm_;
   }
-  // The bins of that order and their count.
+  // The bins of that order and their count: sides 2^sides_log2[a].
+  GridParams bins_grid(const int32_t sides_log2[3], uint64_t* bins) const;
+  GridParams strips_grid(uint64_t* bins) const;
   GridParams rows_grid(uint64_t* bins) const;
   // Copies a sort's permutation into rows_perm_ (the sort buffers are reused).
   void keep_rows_order(const uint32_t* order, int64_t count, cudaStream_t stream);
@@ -199,9 +201,9 @@ class NufftPlan {
   DeviceBuffer tc_parts_, tc_part_start_, tc_packed_;
   int64_t tc_part_upper_bound_ = 0;
 
-  // Tensor-core interpolation (2D f32 type-2 plans of batch >= kTcMinBatch):
-  // the points ordered by exact support start in bins of 8 x 1 cells, their
-  // window records, the slot of every point and the chunk tables.
+  // Tensor-core interpolation of 2D f32 type-2 plans. tcgen05 (64 vectors or
+  // more): the points ordered by exact support start in bins of 8 x 4 cells,
+  // their window records, the slot of every point and the chunk tables.
   bool tc2_enabled_ = false;
   bool tc2_active_ = false;
   GridParams tc2_grid_{};
@@ -209,6 +211,11 @@ class NufftPlan {
   DeviceBuffer tc2_parts_, tc2_part_start_;
   DeviceBuffer tc2_vector_max_;  // batch words: largest grid magnitude of every vector
   int64_t tc2_part_upper_bound_ = 0;
+  // Fewer vectors: the points' strip order (interp_strips.cu) and their
+  // windows in it.
+  bool tc2_strips_ = false;
+  bool strips_for_batch(int batch) const;
+  DeviceBuffer tc2_perm_, tc2_windows_;
 };
 
 }  // namespace b200nufft
