@@ -1342,7 +1342,6 @@ template <typename Complex>
 __global__ void __launch_bounds__(256) fold_dest_kernel(SpreadParams sp, int batch,
                                                         const Complex* __restrict__ scratch,
                                                         const uint32_t* __restrict__ part_start, int64_t part_limit,
-                                                        const int2* __restrict__ candidates,
                                                         Complex* __restrict__ fine) {
   const int slices = sp.tile[2] / kDestCells;
   const uint32_t tile = blockIdx.x / static_cast<uint32_t>(slices);
@@ -1356,41 +1355,34 @@ __global__ void __launch_bounds__(256) fold_dest_kernel(SpreadParams sp, int bat
   const int y = t1 * 16 + static_cast<int>(threadIdx.x >> 4);
   const int z0 = t2 * sp.tile[2] + slice * kDestCells;
   const int n0 = sp.grid.fine[0], n1 = sp.grid.fine[1], n2 = sp.grid.fine[2];
-  // The source tiles of each axis: the candidates of the tile's first cell.
-  int src[3][2];
-  const int first_cell[3] = {t0 * 16, t1 * 16, t2 * sp.tile[2]};
+  // The source tiles of each axis, in the candidates' (ascending) order, and
+  // where they hold the thread's cells: the tile itself and the one before it,
+  // which for the first tile is the last one, a period on (that the candidates
+  // are just these is what dest_fold asserts). -1 where a cell is not covered.
+  const int tiles[3] = {t0, t1, t2};
+  const int n[3] = {n0, n1, n2};
+  int src[3][2], shift[3][2];  // cell - shift: place in the source tile
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const int2* c = candidates + sp.candidate_base[a] + static_cast<int64_t>(first_cell[a]) * sp.candidate_count[a];
-    src[a][0] = c[0].x;
-    src[a][1] = sp.candidate_count[a] > 1 ? c[1].x : -1;
+    const int own = tiles[a], before = own > 0 ? own - 1 : sp.ntiles[a] - 1;
+    const int own_shift = own * sp.tile[a], before_shift = before * sp.tile[a] - (own > 0 ? 0 : n[a]);
+    src[a][0] = own > 0 ? before : own;
+    src[a][1] = own > 0 ? own : before;
+    shift[a][0] = own > 0 ? before_shift : own_shift;
+    shift[a][1] = own > 0 ? own_shift : before_shift;
   }
-  // A cell's local offset in each source tile along an axis; -1 where that
-  // tile does not cover it.
-  auto offsets = [&](int a, int cell, int& o0, int& o1) {
-    o0 = -1;
-    o1 = -1;
-    const int2* c = candidates + sp.candidate_base[a] + static_cast<int64_t>(cell) * sp.candidate_count[a];
-    const int k = sp.candidate_count[a] > 1 ? 2 : 1;
-    for (int i = 0; i < k; ++i) {
-      const int2 e = c[i];
-      if (e.x < 0) break;
-      if (e.x == src[a][0]) o0 = e.y;
-      else if (e.x == src[a][1]) o1 = e.y;
-    }
+  auto place_in = [&](int a, int cell, int u) {
+    const int o = cell - shift[a][u];
+    return cell < n[a] && o < sp.pad[a] ? o : -1;
   };
   const bool xy_inside = x < n0 && y < n1;
-  int ox[2] = {-1, -1}, oy[2] = {-1, -1};
-  if (xy_inside) {
-    offsets(0, x, ox[0], ox[1]);
-    offsets(1, y, oy[0], oy[1]);
-  }
-  int oz[kDestCells][2];
+  int ox[2], oy[2], oz[kDestCells][2];
 #pragma unroll
-  for (int k = 0; k < kDestCells; ++k) {
-    oz[k][0] = -1;
-    oz[k][1] = -1;
-    if (z0 + k < n2) offsets(2, z0 + k, oz[k][0], oz[k][1]);
+  for (int u = 0; u < 2; ++u) {
+    ox[u] = place_in(0, x, u);
+    oy[u] = place_in(1, y, u);
+#pragma unroll
+    for (int k = 0; k < kDestCells; ++k) oz[k][u] = place_in(2, z0 + k, u);
   }
   Complex sum[kDestCells];
 #pragma unroll
@@ -1401,17 +1393,14 @@ __global__ void __launch_bounds__(256) fold_dest_kernel(SpreadParams sp, int bat
   const int plane = sp.pad[0] * sp.pad[1];
 #pragma unroll
   for (int u2 = 0; u2 < 2; ++u2) {
-    if (src[2][u2] < 0) continue;
     bool any_z = false;
 #pragma unroll
     for (int k = 0; k < kDestCells; ++k) any_z = any_z || oz[k][u2] >= 0;
     if (!any_z) continue;  // the same for the whole CTA
 #pragma unroll
     for (int u1 = 0; u1 < 2; ++u1) {
-      if (src[1][u1] < 0) continue;
 #pragma unroll
       for (int u0 = 0; u0 < 2; ++u0) {
-        if (src[0][u0] < 0) continue;
         const int64_t source = src[0][u0] + static_cast<int64_t>(sp.ntiles[0]) *
                                                 (src[1][u1] + static_cast<int64_t>(sp.ntiles[1]) * src[2][u2]);
         const uint32_t first = part_start[source];
@@ -1425,18 +1414,25 @@ __global__ void __launch_bounds__(256) fold_dest_kernel(SpreadParams sp, int bat
           take[k] = covered && oz[k][u2] >= 0;
           at[k] = base + plane * oz[k][u2];
         }
-        for (uint32_t p = first; p < last; ++p) {
-          const Complex* v = scratch + (static_cast<int64_t>(p) * batch + b) * sp.padded_cells;
-          Complex got[kDestCells];
+        // Two parts' loads at a time, added in the parts' order.
+        const int64_t stride = static_cast<int64_t>(batch) * sp.padded_cells;
+        const Complex* v = scratch + (static_cast<int64_t>(first) * batch + b) * sp.padded_cells;
+        for (uint32_t p = first; p < last; p += 2, v += 2 * stride) {
+          const bool pair = p + 1 < last;
+          Complex got[2][kDestCells];
 #pragma unroll
           for (int k = 0; k < kDestCells; ++k) {
-            if (take[k]) got[k] = v[at[k]];
+            if (take[k]) got[0][k] = v[at[k]];
+            if (take[k] && pair) got[1][k] = v[stride + at[k]];
           }
 #pragma unroll
-          for (int k = 0; k < kDestCells; ++k) {
-            if (take[k]) {
-              sum[k].x += got[k].x;
-              sum[k].y += got[k].y;
+          for (int i = 0; i < 2; ++i) {
+#pragma unroll
+            for (int k = 0; k < kDestCells; ++k) {
+              if (take[k] && (i == 0 || pair)) {
+                sum[k].x += got[i][k].x;
+                sum[k].y += got[i][k].y;
+              }
             }
           }
         }
@@ -1579,7 +1575,7 @@ void fold_any(const SpreadParams& sp, int batch, const Complex* scratch, const u
     launch_warp_fold(sp, batch, scratch, part_start, part_limit, candidates, fine, stream);
   } else if (sp.dest_fold && batch < 8) {
     const dim3 grid(static_cast<unsigned>(sp.tile_count * (sp.tile[2] / kDestCells)), static_cast<unsigned>(batch));
-    fold_dest_kernel<Complex><<<grid, 256, 0, stream>>>(sp, batch, scratch, part_start, part_limit, candidates, fine);
+    fold_dest_kernel<Complex><<<grid, 256, 0, stream>>>(sp, batch, scratch, part_start, part_limit, fine);
     note_launch();
   } else if (batch >= 8) {
     launch_fold<8>(sp, batch, scratch, part_start, part_limit, candidates, fine, stream);
