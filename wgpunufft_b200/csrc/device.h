@@ -72,9 +72,10 @@ struct GridParams {
   float horner32[kHornerRows32][kHornerWidth32];
 };
 
-// Prepared windows of `count` f32 points in slot order (coordinates in slot order).
-void prepare_windows(const float* sorted_points, int64_t count, const GridParams& grid, void* windows,
-                     cudaStream_t stream);
+// Prepared windows of `count` f32 points (the caller's coordinates) in the slot
+// order `perm`, and the coordinates in that order where `sorted` is not null.
+void prepare_windows(const float* points, const uint32_t* perm, int64_t count, const GridParams& grid, void* windows,
+                     float* sorted, cudaStream_t stream);
 size_t prepared_window_bytes(int dimensions);
 // inverse[perm[s]] = s for s < count.
 void invert_permutation(const uint32_t* perm, int64_t count, uint32_t* inverse, cudaStream_t stream);
@@ -130,8 +131,6 @@ void reference_bin_order(const uint32_t* perm, const uint32_t* keys, const uint3
                          cudaStream_t stream);
 
 // The coordinates of `count` points in the bin order `perm`.
-void gather_sorted_points(const float* points, const uint32_t* perm, int64_t count, int dimensions,
-                          float* sorted, cudaStream_t stream, StageTimer* timer = nullptr);
 void gather_sorted_points64(const double* points, const uint32_t* perm, int64_t count,
                             int dimensions, double* sorted, cudaStream_t stream,
                             StageTimer* timer = nullptr);

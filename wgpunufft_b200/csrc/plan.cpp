@@ -740,12 +740,10 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       check_cuda(cudaMemcpyAsync(kept, order, static_cast<size_t>(count) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                                  stream),
                  "keep strip order");
-      float* sorted = static_cast<float*>(sorted_points_.reserve(sorted_bytes, "sorted coordinates"));
-      gather_sorted_points(static_cast<const float*>(points), kept, count, dim_, sorted, stream, &timer_);
       StageScope scope(&timer_, kStageBinOffsets, stream);
-      prepare_windows(sorted, count, grid_,
+      prepare_windows(static_cast<const float*>(points), kept, count, grid_,
                       tc2_windows_.reserve(static_cast<size_t>(count) * prepared_window_bytes(dim_), "strip windows"),
-                      stream);
+                      nullptr, stream);
     }
     // The interpolation's own order (rows_grid) is sorted here and its
     // permutation kept; the reference's bins are sorted when they are asked for.
@@ -768,14 +766,16 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       sort_points(static_cast<const float*>(points), count, grid_, KeyKind::ApproximateCell, bins_, buf, offsets,
                   &perm_, &sorted_keys_, stream, &timer_);
     }
-    float* sorted = static_cast<float*>(sorted_points_.reserve(sorted_bytes, "sorted coordinates"));
-    gather_sorted_points(static_cast<const float*>(points), interp_perm(), count, dim_, sorted, stream,
-                         &timer_);
-    // The spreader and interpolator read each point's window start and offset.
+    // The spreader and interpolator read each point's window start and offset;
+    // the coordinates themselves only the tensor-core spreader's preparation
+    // (after this) and a bin order that is asked for later.
+    float* sorted = tc_enabled_ || rows_order_
+                        ? static_cast<float*>(sorted_points_.reserve(sorted_bytes, "sorted coordinates"))
+                        : nullptr;
     void* windows = windows_.reserve(static_cast<size_t>(std::max<int64_t>(count, 1)) * prepared_window_bytes(dim_),
                                      "prepared windows");
     StageScope scope(&timer_, kStageBinOffsets, stream);
-    prepare_windows(sorted, count, grid_, windows, stream);
+    prepare_windows(static_cast<const float*>(points), interp_perm(), count, grid_, windows, sorted, stream);
     if (type_ == 2 && dim_ == 2 && batch_ >= kInterpBinsMinBatch) {
       void* inverse = inverse_.reserve(static_cast<size_t>(std::max<int64_t>(count, 1)) * sizeof(uint32_t),
                                        "point slots");

@@ -570,29 +570,23 @@ __global__ void reference_offsets_kernel(const uint32_t* __restrict__ offsets, i
 
 }  // namespace
 
-void gather_sorted_points(const float* points, const uint32_t* perm, int64_t count, int dimensions,
-                          float* sorted, cudaStream_t stream, StageTimer* timer) {
-  if (count == 0) return;
-  StageScope scope(timer, kStageBinOffsets, stream);
-  const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
-  switch (dimensions) {
-    case 1: gather_points_kernel<1, float><<<blocks, 256, 0, stream>>>(points, perm, count, sorted); break;
-    case 2: gather_points_kernel<2, float><<<blocks, 256, 0, stream>>>(points, perm, count, sorted); break;
-    default: gather_points_kernel<3, float><<<blocks, 256, 0, stream>>>(points, perm, count, sorted); break;
-  }
-  note_launch();
-}
-
 namespace {
 
+// Reads the coordinates through the permutation and keeps them in slot order
+// only where a later kernel reads them (sorted non-null).
 template <int D>
-__global__ void prepare_windows_kernel(const float* __restrict__ sorted, int64_t count, GridParams g,
-                                       PreparedWindow<D>* __restrict__ windows) {
+__global__ void prepare_windows_kernel(const float* __restrict__ points, const uint32_t* __restrict__ perm,
+                                       int64_t count, GridParams g, PreparedWindow<D>* __restrict__ windows,
+                                       float* __restrict__ sorted) {
   const int64_t slot = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (slot >= count) return;
+  const int64_t point = perm[slot];
   float p[D];
 #pragma unroll
-  for (int a = 0; a < D; ++a) p[a] = sorted[slot * D + a];
+  for (int a = 0; a < D; ++a) {
+    p[a] = points[point * D + a];
+    if (sorted != nullptr) sorted[slot * D + a] = p[a];
+  }
   bool reach = true;
 #pragma unroll
   for (int a = 0; a < D; ++a) reach = reach && in_fold_reach(p[a]);
@@ -637,22 +631,22 @@ size_t prepared_window_bytes(int dimensions) {
   return dimensions == 3 ? sizeof(PreparedWindow<3>) : sizeof(PreparedWindow<2>);
 }
 
-void prepare_windows(const float* sorted_points, int64_t count, const GridParams& grid, void* windows,
-                     cudaStream_t stream) {
+void prepare_windows(const float* points, const uint32_t* perm, int64_t count, const GridParams& grid, void* windows,
+                     float* sorted, cudaStream_t stream) {
   if (count == 0) return;
   const unsigned blocks = static_cast<unsigned>((count + 255) / 256);
   switch (grid.dimensions) {
     case 1:
-      prepare_windows_kernel<1><<<blocks, 256, 0, stream>>>(sorted_points, count, grid,
-                                                            static_cast<PreparedWindow<1>*>(windows));
+      prepare_windows_kernel<1><<<blocks, 256, 0, stream>>>(points, perm, count, grid,
+                                                            static_cast<PreparedWindow<1>*>(windows), sorted);
       break;
     case 2:
-      prepare_windows_kernel<2><<<blocks, 256, 0, stream>>>(sorted_points, count, grid,
-                                                            static_cast<PreparedWindow<2>*>(windows));
+      prepare_windows_kernel<2><<<blocks, 256, 0, stream>>>(points, perm, count, grid,
+                                                            static_cast<PreparedWindow<2>*>(windows), sorted);
       break;
     default:
-      prepare_windows_kernel<3><<<blocks, 256, 0, stream>>>(sorted_points, count, grid,
-                                                            static_cast<PreparedWindow<3>*>(windows));
+      prepare_windows_kernel<3><<<blocks, 256, 0, stream>>>(points, perm, count, grid,
+                                                            static_cast<PreparedWindow<3>*>(windows), sorted);
       break;
   }
   note_launch();
