@@ -92,11 +92,14 @@ typedef enum b200nufft_status {
 #define B200NUFFT_MAX_DIMENSIONS 8
 #define B200NUFFT_MAX_TYPE3_DIMENSIONS 3
 
-/* Type-1 spreading engines. AUTO runs 2D f32 type-1 plans of batch >= 16 on
- * the tensor cores (3xTF32 tcgen05 MMAs) when their active batch is at least
- * 16 and the chosen bins allow it, and everything else on the CUDA cores.
- * TENSOR_CORES asks for the tensor cores whenever the plan qualifies
- * (plan creation fails otherwise); CUDA_CORES never uses them. */
+/* Spreading and interpolation engines of f32 plans. AUTO runs 2D f32 plans of
+ * batch >= 16 on the tensor cores (3xTF32 tcgen05 MMAs, or mma.sync products)
+ * when their active batch is at least 16 and the chosen bins allow it, crowded
+ * 3D tiles and 2D tiles of width 7 as mma.sync products in split tf32, and
+ * everything else on the CUDA cores. TENSOR_CORES asks for the batched
+ * tensor-core paths whenever the plan qualifies (plan creation fails
+ * otherwise); CUDA_CORES never uses tensor cores for f32 sums. f64 plans use
+ * f64 matrix instructions, which round as fused multiply-adds, either way. */
 #define B200NUFFT_SPREAD_AUTO 0
 #define B200NUFFT_SPREAD_CUDA_CORES 1
 #define B200NUFFT_SPREAD_TENSOR_CORES 2
@@ -208,10 +211,10 @@ int b200nufft_encode(b200nufft_plan plan, int64_t active_batch, int64_t point_co
  * `permutation` (device, point_count words) receives the original index of
  * every slot and `bin_offsets` (device, bin_count + 1 words) the first slot of
  * every bin followed by the total (NdPointBins::encode,
- * src/gpu_nd_bins.rs:336-471). Either pointer may be null. 3D type-2 plans
- * interpolate in another order and sort the bin order at the first call after
- * each set_points, on `stream` (it reserves a device buffer of 3 coordinates
- * per point the first time). */
+ * src/gpu_nd_bins.rs:336-471). Either pointer may be null. 3D type-2
+ * plans, and 2D f64 ones of eps below 1e-3, interpolate in another order and
+ * sort the bin order at the first call after each set_points, on `stream` (3D
+ * plans reserve a device buffer of 3 coordinates per point the first time). */
 int b200nufft_copy_bin_order(b200nufft_plan plan, uint32_t *permutation,
                              uint32_t *bin_offsets, void *stream);
 

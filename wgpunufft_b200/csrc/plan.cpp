@@ -128,6 +128,7 @@ NufftPlan::NufftPlan(const b200nufft_config& c, bool with_device) : has_device_(
     throw NufftFailure{B200NUFFT_INVALID_ARGUMENT,
                        "tensor cores need a 2D f32 plan with a window of at most 8 points (type 1) or 7 (type 2)"};
   }
+  cuda_cores_only_ = c.spread_method == B200NUFFT_SPREAD_CUDA_CORES;
   const bool tc_requested = (c.spread_method == B200NUFFT_SPREAD_AUTO && batch_ >= kTcMinBatch) ||
                             c.spread_method == B200NUFFT_SPREAD_TENSOR_CORES;
   tc_enabled_ = tc1_qualifies && tc_requested;
@@ -494,7 +495,8 @@ void NufftPlan::configure_tiles() {
       sp.warp_segments = static_cast<const uint32_t*>(warp_segments_.get());
     }
   }
-  if (dim_ == 3 && precision_ == B200NUFFT_PRECISION_F32 && w >= kStripMinWidth && w <= kStripMaxWidth) {
+  sp.products = precision_ == B200NUFFT_PRECISION_F32 && !cuda_cores_only_ ? 1 : 0;
+  if (dim_ == 3 && sp.products != 0 && w >= kStripMinWidth && w <= kStripMaxWidth) {
     spread_strip_layout(sp.pad, sp.strip_pitch0, sp.strip_pitch01);
   }
   // Parts of at most kPartCap records (f64), fewer for small point sets so that
@@ -536,7 +538,10 @@ void NufftPlan::configure_tiles() {
     sp.cap_bins = bins_;
     records_per_cap = std::max<int64_t>(most_ctas, (std::max<int64_t>(point_count_, 0) + part_cap - 1) / part_cap);
   }
-  const int64_t part_bound = type_ == 1 ? sp.tile_count + tiles_per_bin * records_per_cap + 1
+  // (A part but for a tile's last holds at least 256 records.)
+  const int64_t full_parts =
+      std::min(tiles_per_bin * records_per_cap, tiles_per_bin * std::max<int64_t>(point_count_, 0) / 256);
+  const int64_t part_bound = type_ == 1 ? sp.tile_count + full_parts + 1
                                         : sp.tile_count + (std::max<int64_t>(point_count_, 0) * tiles_per_bin +
                                                            sp.part_cap - 1) / sp.part_cap + 1;
   // Candidate (tile, local) pairs of every coordinate of every axis: tile t
@@ -1319,7 +1324,9 @@ void NufftPlan::spread_to(int64_t active_batch, const void* strengths, void* gri
 }
 
 bool NufftPlan::interp_strips() const {
-  return interp_strips_chosen(dim_, precision_ != B200NUFFT_PRECISION_F32, kernel_.width, point_count_, fine_count_);
+  const bool f64 = precision_ != B200NUFFT_PRECISION_F32;
+  return (f64 || !cuda_cores_only_) &&
+         interp_strips_chosen(dim_, f64, kernel_.width, point_count_, fine_count_);
 }
 
 bool NufftPlan::strips_for_batch(int batch) const {

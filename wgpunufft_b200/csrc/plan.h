@@ -205,6 +205,7 @@ class NufftPlan {
   // more): the points ordered by exact support start in bins of 8 x 4 cells,
   // their window records, the slot of every point and the chunk tables.
   bool tc2_enabled_ = false;
+  bool cuda_cores_only_ = false;  // spread method CUDA_CORES: no f32 matrix products
   bool tc2_active_ = false;
   GridParams tc2_grid_{};
   DeviceBuffer tc2_offsets_, tc2_weights_, tc2_inverse_, tc2_tile_chunks_, tc2_tile_chunk_start_, tc2_chunks_;

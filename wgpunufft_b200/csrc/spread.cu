@@ -970,7 +970,7 @@ __device__ __forceinline__ void spread_part(
   const bool bucket = warp_path && record_end - record_begin <= static_cast<uint32_t>(kWarpMaxRecords) &&
                       (tile_cells + 1) * kSpreadWarps <= T::kWordsPerCell * span &&
                       tile_total >= static_cast<uint32_t>(tile_cells);
-  const bool row_path = kRowCapable && sp.tile[0] <= kRowMaxTile && (1 << sp.grid.axis[1].shift) <= 9 - W &&
+  const bool row_path = kRowCapable && sp.products != 0 && sp.tile[0] <= kRowMaxTile && (1 << sp.grid.axis[1].shift) <= 9 - W &&
                         2 * tile_total >= static_cast<uint32_t>(tile_cells);
   // (A warp's register sums hold at most 2^11 records of magnitude below
   // 2^27: below 2^38, which add_split takes.)

@@ -49,6 +49,8 @@ struct SpreadParams {
   int32_t pitch01;
   int32_t span;
   const uint32_t* warp_segments;
+  // f32 plans that may use the tensor cores (spread method not CUDA_CORES).
+  int32_t products;
   // 3D f32 plans of widths kStripMinWidth..kStripMaxWidth: pitches of the
   // padded tile under the tensor-core strips (spread_strip_layout).
   int32_t strip_pitch0;
