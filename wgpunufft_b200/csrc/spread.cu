@@ -1589,16 +1589,16 @@ void launch_spread_width(const SpreadParams& sp, const SpreadLaunchT<T>& l, cuda
   if constexpr (D == 3 && sizeof(typename T::Real) == 8 && W >= kReg64MinWidth && W <= kReg64MaxWidth) {
     throw NufftFailure{B200NUFFT_INTERNAL, "3D f64 plans of this width spread in registers"};
   } else {
-  const size_t smem = spread_tile_bytes<D, W, T>(sp) + spread_aux_bytes<D, W, T>();
-  auto kernel = spread_tiles_kernel<D, W, T>;
-  check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)),
-             "spread shared memory");
-  const dim3 grid(static_cast<unsigned>(l.part_upper_bound), static_cast<unsigned>(l.batch));
-  kernel<<<grid, kSpreadThreads, smem, stream>>>(sp, l.points, l.windows, l.strengths, l.point_count, l.batch,
-                                                 l.perm, l.offsets, l.part_start, l.max_bits,
-                                                 l.scratch);
-  note_launch();
+    const size_t smem = spread_tile_bytes<D, W, T>(sp) + spread_aux_bytes<D, W, T>();
+    auto kernel = spread_tiles_kernel<D, W, T>;
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(smem)),
+               "spread shared memory");
+    const dim3 grid(static_cast<unsigned>(l.part_upper_bound), static_cast<unsigned>(l.batch));
+    kernel<<<grid, kSpreadThreads, smem, stream>>>(sp, l.points, l.windows, l.strengths, l.point_count, l.batch,
+                                                   l.perm, l.offsets, l.part_start, l.max_bits,
+                                                   l.scratch);
+    note_launch();
   }
 }
 
