@@ -170,3 +170,23 @@ def test_batched_2d_type2_strips_match_the_gather(eps, batch, n_modes, spread):
         return out.cpu().numpy()
 
     assert rel(run(w.SpreadMethod.TENSOR_CORES), run(w.SpreadMethod.CUDA_CORES)) < F32_ROUNDING
+
+
+@pytest.mark.parametrize("tile", [1, 2, 4, 64])
+def test_2d_f64_strips_of_every_tuned_tile(tile):
+    """Tiles from one start up: the records' counters then outgrow the tile's cells."""
+    import wgpunufft_b200 as w
+    from wgpunufft_b200 import _native
+
+    eps, n_modes, count = 1e-4, (12, 17), 900  # width 5
+    rng = np.random.default_rng(16)
+    points = points_of(rng, "crowded", count, [2 * n for n in n_modes]).astype(np.float64)
+    inputs = values(rng, 2, count).astype(np.complex128)
+    override = _native.library().b200nufft_tuning_override
+    override(_native.Tuning(tile, 0, 0, 0))
+    try:
+        _, got = transform(w, 1, n_modes, eps, w.Precision.F64, 2, points, inputs, int(np.prod(n_modes)))
+    finally:
+        override(None)
+    for b in range(2):
+        assert rel(got[b], native.direct_type1(points, inputs[b], n_modes)[0]) < 20 * eps

@@ -808,7 +808,14 @@ __host__ __device__ inline size_t spread_tile_bytes(const SpreadParams& sp) {
   int span = sp.padded_cells;
   if (warp_capable<D, W, T>() && sp.span > span) span = sp.span;
   if (strip_capable<D, W, T>() && sp.strip_pitch01 * sp.pad[2] > span) span = sp.strip_pitch01 * sp.pad[2];
-  return static_cast<size_t>(T::kWordsPerCell) * span * sizeof(typename T::Word);
+  size_t bytes = static_cast<size_t>(T::kWordsPerCell) * span * sizeof(typename T::Word);
+  // The 2D f64 strips order their records with counters in the tile's place,
+  // which in a tile of one start (w 5) take more than its cells.
+  if (D == 2 && sizeof(typename T::Real) == 8 && strip_capable<D, W, T>()) {
+    const size_t counters = strip_counter_bytes(strip64_count<W>(sp.tile[0], sp.tile[1]), kStrip64X);
+    if (counters > bytes) bytes = counters;
+  }
+  return bytes;
 }
 template <int D, int W, typename T>
 __host__ __device__ constexpr size_t spread_aux_bytes() {
@@ -1815,6 +1822,35 @@ void batch_spread(const BatchProblem* problems, const BatchStrengths& strengths,
 
 void spread_fold(const SpreadParams& sp, const SpreadLaunch& l, cudaStream_t stream) {
   fold_any(sp, l.batch, l.scratch, l.part_start, l.part_upper_bound, l.candidates, l.fine, stream);
+}
+
+extern "C" int64_t b200nufft_internal_strip64_tile_bytes(int32_t width, int32_t tile0, int32_t tile1) {
+  SpreadParams sp{};
+  const int32_t tile[3] = {tile0, tile1, 1};
+  sp.padded_cells = 1;
+  for (int a = 0; a < 3; ++a) {
+    sp.tile[a] = tile[a];
+    sp.pad[a] = a < 2 ? tile[a] + width - 1 : 1;
+    sp.padded_cells *= sp.pad[a];
+  }
+  switch (width) {
+#define B200NUFFT_STRIP64_CASE(WIDTH) \
+  case WIDTH: return static_cast<int64_t>(spread_tile_bytes<2, WIDTH, F64Traits>(sp));
+    B200NUFFT_STRIP64_CASE(5)
+    B200NUFFT_STRIP64_CASE(6)
+    B200NUFFT_STRIP64_CASE(7)
+    B200NUFFT_STRIP64_CASE(8)
+    B200NUFFT_STRIP64_CASE(9)
+    B200NUFFT_STRIP64_CASE(10)
+    B200NUFFT_STRIP64_CASE(11)
+    B200NUFFT_STRIP64_CASE(12)
+    B200NUFFT_STRIP64_CASE(13)
+    B200NUFFT_STRIP64_CASE(14)
+    B200NUFFT_STRIP64_CASE(15)
+    B200NUFFT_STRIP64_CASE(16)
+#undef B200NUFFT_STRIP64_CASE
+    default: return 0;
+  }
 }
 
 size_t spread_shared_bytes(const SpreadParams& sp) {

@@ -102,6 +102,8 @@ constexpr int kStripMaxWidth = 7;
 // 2D f64 windows without register runs (spread_run) always take the strips.
 constexpr int kStrip64MinWidth = 5;
 constexpr int kStripMaxRecords = 2048;  // records of a part under the strips, at most
+// For tests: bytes a 2D f64 strip tile of tile0 x tile1 starts takes in shared memory.
+extern "C" int64_t b200nufft_internal_strip64_tile_bytes(int32_t width, int32_t tile0, int32_t tile1);
 // Pitches of the padded tile (pad[a] cells, some slack allowed) that spread
 // a strip's flush, 8 rows x 4 even planes per warp, over the most banks.
 void spread_strip_layout(const int32_t pad[3], int32_t& pitch0, int32_t& pitch01);

@@ -39,10 +39,15 @@ struct StripShared {
   float* stage;
 };
 
+// Bytes of strip_order's counters.
+__host__ __device__ constexpr size_t strip_counter_bytes(int strips, int per_strip) {
+  return sizeof(uint32_t) * kSpreadWarps * (static_cast<size_t>(strips) * per_strip + 1);
+}
+
 // Orders the part's records by key, stably: key_of(load_of(slot)) lies in
 // [0, strips * per_strip), or is negative for a record to skip. Fills sh.sorted
 // with slots and sh.start[0, strips]. `count` is scratch of
-// (strips * per_strip + 1) * kSpreadWarps words. The caller synchronizes.
+// strip_counter_bytes(strips, per_strip). The caller synchronizes.
 template <typename LoadOf, typename KeyOf>
 __device__ __forceinline__ void strip_order(const uint32_t* row_begin, const uint32_t* row_prefix, int rows,
                                             uint32_t record_begin, uint32_t record_end, int strips, int per_strip,
@@ -602,6 +607,10 @@ struct Strip64 {
   static constexpr int kRows = W + 3 < kMaxHornerCoefficients ? W + 3 : kMaxHornerCoefficients;
   static constexpr int kTaps = (W + 3) / 4 * 2;
 };
+template <int W>
+__host__ __device__ constexpr int strip64_count(int t0, int t1) {
+  return ((t0 + kStrip64X - 1) / kStrip64X) * ((t1 + Strip64<W>::S - 1) / Strip64<W>::S);
+}
 
 template <int W>
 __device__ void spread_strips2_f64(const SpreadParams& sp, const double2* points, const double2* sv,
