@@ -17,6 +17,14 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// The tensor core cuts a sum of products off at 24 bits instead of rounding it:
+// half a unit of the last place towards zero on average, over mantissas of
+// uniform logarithm 2^-24 / (2 ln 2) of the sum. All sums of a cell lose this
+// share of their magnitude alike, so f32 strips of one-signed strengths came
+// out 4e-8 too small (radial 128^3, w 6: error against 64 bits 1.29e-7 with
+// scalar multiply-adds, 1.40e-7 with the products).
+constexpr float kProductLoss = 4.3e-8f;
+
 // v to the nearest value of the 19 bits a tf32 operand keeps, and the exact
 // remainder, whose sign is then independent of v's: what the products drop
 // (the remainder's own last bits, low times low) does not add up.

@@ -1202,7 +1202,8 @@ __device__ __forceinline__ void spread_part(
   __syncthreads();
   typename T::Complex* out = scratch + (static_cast<int64_t>(part) * batch + b) * padded;
   // The strips' low words are signed sums, below 2^24 as the high words of
-  // all but extreme cells: one rounding.
+  // all but extreme cells: one rounding. Their products' truncation is made
+  // good here (kProductLoss).
   const float down_lo = T::kPreparedWindows ? ldexpf(1.0f, -S / 2) : 0.0f;
   const float down_hi = T::kPreparedWindows ? ldexpf(1.0f, -S - (-S / 2)) : 0.0f;
   auto value = [&](int which, int at) {
@@ -1210,7 +1211,7 @@ __device__ __forceinline__ void spread_part(
       if (strip_path || row_path) {
         const float lo = static_cast<float>(static_cast<int32_t>(acc[(2 * which) * span + at]));
         const float hi = static_cast<float>(static_cast<int32_t>(acc[(2 * which + 1) * span + at]));
-        return fmaf(hi, 65536.0f, lo) * down_lo * down_hi;
+        return fmaf(hi, 65536.0f, fmaf(hi, 65536.0f * kProductLoss, lo)) * down_lo * down_hi;
       }
     }
     return T::value(acc, span, which, at, S);
