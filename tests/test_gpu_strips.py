@@ -11,7 +11,7 @@ compared with the direct sums at the reference's 20 eps (2D) and 32 eps (3D).
 import numpy as np
 import pytest
 
-from oracle import native
+from oracle import gpu_direct, native
 
 pytestmark = pytest.mark.gpu
 
@@ -219,3 +219,29 @@ def test_f32_products_lose_no_share_of_one_signed_sums(eps, n_modes):
         got, want = outs
         shares.append(float((got * want.conj()).real.sum() / (want.abs() ** 2).sum()) - 1.0)
     assert abs(np.mean(shares)) < 2e-8
+
+
+@pytest.mark.parametrize("eps", [1e-4, 1e-5, 1e-6, 1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-12, 1e-13, 1e-14])
+@pytest.mark.parametrize("n_modes, spread", [((70, 90), "uniform"), ((12, 150), "edges")])
+def test_2d_f64_values_do_not_depend_on_the_other_points(eps, n_modes, spread):
+    """A few scattered points, which each lane of a warp gathers, and the same
+    points among many, which go through the products: the same bits."""
+    import torch
+
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(17)
+    few = points_of(rng, spread, 401, [2 * n for n in n_modes]).astype(np.float64)
+    many = rng.uniform(-np.pi, np.pi, (90_000, 2))
+    inputs = torch.from_numpy(values(rng, 6, int(np.prod(n_modes))).astype(np.complex128)).cuda()
+
+    def run(points):
+        plan = w.NufftPlan.type2_gpu(w.NufftConfig(n_modes, eps, batch=6, precision=w.Precision.F64))
+        out = torch.empty((6, len(points)), dtype=torch.complex128, device="cuda")
+        plan.encode_type2_gpu(torch.from_numpy(points).cuda(), inputs, out)
+        plan.synchronize()
+        return out
+
+    alone = run(few)
+    among = run(np.concatenate([few, many]))[:, : len(few)].contiguous()
+    assert torch.equal(torch.view_as_real(alone), torch.view_as_real(among))

@@ -65,8 +65,59 @@ struct F64Strips {
   static constexpr int kWarps = 2;
 };
 
+// Groups of a warp's 32 points, at most, that the 2D f64 products serve; beyond
+// that each lane gathers its own w^2 cells, adding them in the products' order
+// (the same bits). A group's products cost a half (w 5) to a fifth (w 13) of 32
+// gathers. 1024^2 modes, uniform, us per transform with products alone and so: w 7,
+// 1/16 point per cell 195 / 139, 1/4 244 / 224, one point 392 / 401; w 13, 1/16
+// 249 / 221, one point 614 / 626.
+template <int W>
+constexpr int kMostGroups = W <= 6 ? 1 : (W <= 8 ? 2 : (W - 1) / 2);
+
+// One point's w^2 cells, added in the products' order: down the rows, then
+// along the columns of one residue modulo 4, as the four lanes of a product do.
+// A call, so that the products keep their registers.
+template <int W>
+__device__ __noinline__ void gather_columns(const double* wx, const double* wy, int x0, int y0, int n0, int n1,
+                                            const double2* grid, int64_t grid_stride, int vectors, double2* output,
+                                            int64_t output_stride) {
+  for (int b = 0; b < vectors; ++b, grid += grid_stride, output += output_stride) {
+    double2 columns[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) columns[i] = make_double2(0.0, 0.0);
+#pragma unroll 2
+    for (int j = 0; j < W; ++j) {
+      const int y = y0 + j >= n1 ? y0 + j - n1 : y0 + j;
+      const double2* const row = grid + static_cast<int64_t>(y) * n0;
+      const double weight = wy[j];
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        const int x = x0 + i >= n0 ? x0 + i - n0 : x0 + i;
+        columns[i] = cfma(__ldg(row + x), weight, columns[i]);
+      }
+    }
+    double2 v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) v[t] = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const int residue = (x0 + i) & 3;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (residue == t) v[t] = cfma(columns[i], wx[i], v[t]);
+      }
+    }
+    *output = make_double2((v[0].x + v[2].x) + (v[1].x + v[3].x), (v[0].y + v[2].y) + (v[1].y + v[3].y));
+  }
+}
+
+// CTAs of an SM that the registers are held to (2D f64: what the products alone
+// take, so that the gathers do not cost them their occupancy; 0: free).
+template <int D, int W, typename T>
+constexpr int kMinBlocks = D == 2 && sizeof(typename T::Real) == 8 ? (W <= 9 ? 10 : 8) : 0;
+
 template <int D, int W, int V, typename T>
-__global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
+__global__ void __launch_bounds__(T::kWarps * 32, (kMinBlocks<D, W, T>)) interp_strips_kernel(
     GridParams grid, const typename T::Real* __restrict__ points, const void* __restrict__ windows, int64_t count,
     const uint32_t* __restrict__ perm, const typename T::Complex* __restrict__ fine, int batch,
     typename T::Complex* __restrict__ output) {
@@ -170,6 +221,39 @@ __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
   }
   __syncwarp();
 
+  const int strip_y = start[1] >> S::kShiftY, strip_z = D == 3 ? start[2] >> S::kShiftZ : 0;
+  unsigned todo = __ballot_sync(0xFFFFFFFFu, reach);
+  // The lanes of the next group: one strip, x starts within kSpan cells.
+  struct Group {
+    int x, y, z;
+    bool mine;
+    unsigned members;
+  };
+  auto next_group = [&](unsigned left) {
+    const int leader = __ffs(left) - 1;
+    Group q;
+    q.x = __shfl_sync(0xFFFFFFFFu, start[0], leader);
+    q.y = __shfl_sync(0xFFFFFFFFu, strip_y, leader);
+    q.z = D == 3 ? __shfl_sync(0xFFFFFFFFu, strip_z, leader) : 0;
+    q.mine = ((left >> lane) & 1u) && strip_y == q.y && strip_z == q.z && start[0] >= q.x && start[0] < q.x + kSpan;
+    q.members = __ballot_sync(0xFFFFFFFFu, q.mine);
+    return q;
+  };
+  if constexpr (F64 && D == 2) {
+    // Points too far apart for products: every lane gathers its own.
+    int groups = 0;
+    for (unsigned left = todo; left != 0u && groups <= kMostGroups<W>; ++groups) left &= ~next_group(left).members;
+    if (groups > kMostGroups<W>) {
+      if (reach) {
+        gather_columns<W>(st.wx + lane * S::kPitchX,
+                          st.wy + lane * S::kPitchY + (start[1] & ((1 << S::kShiftY) - 1)), start[0], start[1], n0, n1,
+                          fine + first_vector * grid.fine_count, grid.fine_count, last_vector - first_vector,
+                          output + first_vector * count + point, count);
+      }
+      return;
+    }
+  }
+
   // Fragments: lane (g, t) holds rows (points) 8 m + g, and columns
   // x = 4 n + t (real and imaginary part) of the products.
   const int g = lane >> 2, t = lane & 3;
@@ -198,16 +282,12 @@ __global__ void __launch_bounds__(T::kWarps * 32) interp_strips_kernel(
       for (int k = 0; k < K; ++k) a64[m][k] = st.wy[(8 * m + g) * S::kPitchY + 4 * k + t];
     }
   }
-  const int strip_y = start[1] >> S::kShiftY, strip_z = D == 3 ? start[2] >> S::kShiftZ : 0;
-  unsigned todo = __ballot_sync(0xFFFFFFFFu, reach);
   while (todo != 0u) {
-    const int leader = __ffs(todo) - 1;
-    const int lx = __shfl_sync(0xFFFFFFFFu, start[0], leader);
-    const int ly = __shfl_sync(0xFFFFFFFFu, strip_y, leader);
-    const int lz = D == 3 ? __shfl_sync(0xFFFFFFFFu, strip_z, leader) : 0;
-    const bool mine = ((todo >> lane) & 1u) && strip_y == ly && strip_z == lz && start[0] >= lx &&
-                      start[0] < lx + kSpan;
-    const unsigned members = __ballot_sync(0xFFFFFFFFu, mine);
+    const Group group = next_group(todo);
+    const int lx = group.x, ly = group.y;
+    [[maybe_unused]] const int lz = group.z;
+    const bool mine = group.mine;
+    const unsigned members = group.members;
     todo &= ~members;
     const int hx = __reduce_max_sync(0xFFFFFFFFu, mine ? start[0] : lx) + W - 1;
     // Blocks of columns that the windows of each 16 points reach (3D f32: one
