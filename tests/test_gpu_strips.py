@@ -245,3 +245,22 @@ def test_2d_f64_values_do_not_depend_on_the_other_points(eps, n_modes, spread):
     alone = run(few)
     among = run(np.concatenate([few, many]))[:, : len(few)].contiguous()
     assert torch.equal(torch.view_as_real(alone), torch.view_as_real(among))
+
+
+@pytest.mark.parametrize("eps", [1e-4, 1e-5, 1e-6, 1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-12, 1e-13, 1e-14])
+@pytest.mark.parametrize("n_modes", [(40, 50), (400, 400)])  # one kernel; a kernel for sparse tiles, one for others
+def test_2d_f64_sparse_and_crowded_tiles(eps, n_modes):
+    """Scattered points and a few crowds in one set, three vectors."""
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(18)
+    fine = np.asarray([2 * n for n in n_modes])
+    count = int(fine.prod()) // 160
+    crowds = [c + 2 * np.pi / fine * rng.normal(0.0, 6.0, (600, 2)) for c in ((0.0, 0.0), (-np.pi, 2.0))]
+    points = np.concatenate([rng.uniform(-np.pi, np.pi, (count, 2)), *crowds])
+    points = np.remainder(points + np.pi, 2 * np.pi) - np.pi
+    inputs = values(rng, 3, len(points)).astype(np.complex128)
+    plan, got = transform(w, 1, n_modes, eps, w.Precision.F64, 3, points, inputs, int(np.prod(n_modes)))
+    want = gpu_direct.direct_type1(points, inputs, n_modes)
+    for b in range(3):
+        assert rel(got[b], want[b]) < max(20 * eps, 2e-13)

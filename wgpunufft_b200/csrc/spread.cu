@@ -119,9 +119,6 @@ struct F64Traits {
   static __device__ __forceinline__ void add(Word* acc, int padded, int part, int c, double value) {
     atomicAdd(&acc[part * padded + c], static_cast<unsigned long long>(__double2ll_rn(value)));
   }
-  static __device__ __forceinline__ double value(const Word* acc, int padded, int part, int c, int S) {
-    return ldexp(__ll2double_rn(static_cast<long long>(acc[part * padded + c])), -S);
-  }
 };
 
 template <typename T>
@@ -716,8 +713,111 @@ __device__ void spread_warp3(const SpreadParams& sp, const PreparedWindow<3>* wi
   if (run >= 0) flush();
 }
 
-// Tiles that take the strips: 3D f32 tiles of enough records, all 2D f64
-// tiles of windows without register runs.
+// 2D f64 tiles of too few records for the strips (kStrip64CellsPerRecord) are
+// spread by whole warps, one record at a time: lanes 0 .. 2w-1
+// evaluate one window tap each (axis a = lane / w), and lane l owns the
+// window cells u = l + 32 q (x = u mod w, y = u / w), summing a run of
+// records with one support start in f64 registers in record order. A run
+// reaches the 64-bit fixed-point tile once, when its start changes; the tile
+// of a part of at most 4096 records stays below 2^62 in every cell whatever
+// the runs, so the scale is the record-by-record one.
+template <int W>
+__device__ void spread_warp2_f64(const SpreadParams& sp, const double* points, const double2* sv,
+                                 const uint32_t* perm, const uint32_t* row_begin, const uint32_t* row_prefix,
+                                 int rows, const int* origin, uint32_t record_begin, uint32_t record_end,
+                                 unsigned long long* acc, int padded, double (*stage)[2][W], const double* table,
+                                 double scale_lo, double scale_hi) {
+  using L = Strip64<W>;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int R = (W * W + 31) / 32;
+  double ar[R], ai[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) ar[q] = ai[q] = 0.0;
+  int run_x = -1, run_y = 0;
+  const int pad0 = sp.pad[0];
+  auto flush = [&]() {
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int u = lane + 32 * q;
+      if (u < W * W) {
+        const int c = (run_y + u / W) * pad0 + run_x + u % W;
+        F64Traits::add(acc, padded, 0, c, ar[q]);
+        F64Traits::add(acc, padded, 1, c, ai[q]);
+      }
+      ar[q] = ai[q] = 0.0;
+    }
+  };
+  // Warp w spreads the consecutive records [warp_begin, warp_end).
+  const uint32_t n = record_end - record_begin;
+  const uint32_t per_warp = (n + kSpreadWarps - 1) / kSpreadWarps;
+  const uint32_t warp_begin = record_begin + min(n, per_warp * warp);
+  const uint32_t warp_end = record_begin + min(n, per_warp * (warp + 1));
+  const int axis = lane < W ? 0 : 1, tap = lane < W ? lane : lane - W;
+  double* my_tap = &stage[warp][axis][tap];
+  int row = 0;
+  // Coordinates and strengths are loaded one record ahead, point indexes two.
+  double next_x = 0.0, next_y = 0.0;
+  double2 next_c = make_double2(0.0, 0.0);
+  uint32_t next_point = 0;
+  auto load_slot = [&](uint32_t r, uint32_t& slot) {
+    if (r < warp_end) slot = record_slot(r, row, row_begin, row_prefix, rows);
+    return r < warp_end;
+  };
+  uint32_t slot = 0;
+  if (load_slot(warp_begin, slot)) {
+    next_x = points[static_cast<int64_t>(slot) * 2];
+    next_y = points[static_cast<int64_t>(slot) * 2 + 1];
+    next_c = sv[perm[slot]];
+  }
+  if (load_slot(warp_begin + 1, slot)) next_point = perm[slot];
+  for (uint32_t r = warp_begin; r < warp_end; ++r) {
+    const double x = next_x, y = next_y;
+    const double2 c = next_c;
+    if (r + 1 < warp_end) {
+      next_x = points[static_cast<int64_t>(slot) * 2];
+      next_y = points[static_cast<int64_t>(slot) * 2 + 1];
+      next_c = sv[next_point];
+      if (load_slot(r + 2, slot)) next_point = perm[slot];
+    }
+    if (!F64Traits::in_reach(x) || !F64Traits::in_reach(y)) continue;
+    int32_t start[2];
+    double offset[2];
+    support_of64(x, sp.grid.axis64[0], sp.grid.half_width64, start[0], offset[0]);
+    support_of64(y, sp.grid.axis64[1], sp.grid.half_width64, start[1], offset[1]);
+    const int lx = wrap_start(start[0], sp.grid.axis[0].length) - origin[0];
+    const int ly = wrap_start(start[1], sp.grid.axis[1].length) - origin[1];
+    if (lx < 0 || lx >= sp.tile[0] || ly < 0 || ly >= sp.tile[1]) continue;  // another tile owns it
+    __syncwarp();  // the previous record's taps are read
+    if (lane < 2 * W) {
+      const double local = 2.0 * (axis == 0 ? offset[0] : offset[1]) + static_cast<double>(W - 1);
+      const double* coefficients = table + (tap & 1) * L::kTaps + tap / 2;
+      double v = 0.0;
+#pragma unroll
+      for (int r = 0; r < L::kRows; ++r) v = fma(v, local, coefficients[r * 2 * L::kTaps]);
+      *my_tap = fabs(local) <= 1.0 ? v : 0.0;
+    }
+    __syncwarp();
+    if (lx != run_x || ly != run_y) {
+      if (run_x >= 0) flush();
+      run_x = lx;
+      run_y = ly;
+    }
+    const double sr = (c.x * scale_lo) * scale_hi, si = (c.y * scale_lo) * scale_hi;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int u = lane + 32 * q;
+      if (u < W * W) {
+        const double weight = stage[warp][0][u % W] * stage[warp][1][u / W];
+        ar[q] = fma(sr, weight, ar[q]);
+        ai[q] = fma(si, weight, ai[q]);
+      }
+    }
+  }
+  if (run_x >= 0) flush();
+}
+
+// Tiles that can take the strips: 3D f32 tiles, and 2D f64 tiles of windows
+// without register runs, where they hold enough records.
 template <int D, int W, typename T>
 __host__ __device__ constexpr bool strip_capable() {
   if (sizeof(typename T::Real) == 8) return D == 2 && W >= kStrip64MinWidth;
@@ -859,22 +959,14 @@ __device__ __forceinline__ void spread_part(
   __shared__ int64_t s_tile;
   __shared__ uint32_t warp_totals[kSpreadThreads / 32];
 
-  const uint32_t total_parts = part_start[sp.tile_count];
-  if (part >= total_parts) return;
+  if (part >= part_start[sp.tile_count]) return;
+  // (Loaded ahead of the waits below: each would add a load's latency to the CTA.)
+  const uint32_t part_cap = static_cast<uint32_t>(part_cap_of(sp));
+  const typename T::Bits scale_bits = max_bits[b];
   const int tid = threadIdx.x;
   if (tid < 32) {
-    // Last tile whose first part is at or below `part`: a warp narrows the
-    // range 33-fold per step (dependent loads, on every CTA's critical path).
-    int64_t low = 0, count = sp.tile_count;  // the tile lies in [low, low + count)
-    while (count > 1) {
-      const int64_t step = (count + 32) / 33;
-      const int64_t probe = low + (tid + 1) * step;
-      const bool below = probe < low + count && part_start[probe] <= part;
-      const int passed = __popc(__ballot_sync(0xFFFFFFFFu, below));
-      count = min(step, count - passed * step);
-      low += passed * step;
-    }
-    if (tid == 0) s_tile = low;
+    const int64_t found = part_tile(part_start, sp.tile_count, part);
+    if (tid == 0) s_tile = found;
   }
   const int padded = sp.padded_cells;
   // The shared tile: dense (span = padded) or with the warp path's pitches.
@@ -888,7 +980,12 @@ __device__ __forceinline__ void spread_part(
     const int units = static_cast<int>(T::kWordsPerCell * sizeof(Word) / 16) * span;
     for (int c = tid; c < units; c += kSpreadThreads) acc16[c] = make_uint4(0u, 0u, 0u, 0u);
   };
-  if constexpr (!strip_capable<D, W, T>()) clear_tile();
+  // (2D f64 strips clear it again, over their record counters.)
+  constexpr bool kStripCapable = strip_capable<D, W, T>();
+  constexpr bool kStrip64 = kStripCapable && sizeof(Real) == 8;
+  if constexpr (!kStripCapable || kStrip64) clear_tile();
+  __shared__ __align__(16) double table[kStrip64 ? Strip64<W>::kRows * 2 * Strip64<W>::kTaps : 1];
+  if constexpr (kStrip64) strip64_table<W>(sp.grid, table);
   __syncthreads();
   const int64_t tile = s_tile;
   const uint32_t part_in_tile = part - part_start[tile];
@@ -896,12 +993,12 @@ __device__ __forceinline__ void spread_part(
   // Tile origin and bin rows.
   int origin[3], bin_lo[3], bin_hi[3], rows_along[3];
   {
-    int64_t rest = tile;
+    uint32_t rest = static_cast<uint32_t>(tile);  // parts and tiles count in 32 bits
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-      const int64_t ta = rest % sp.ntiles[a];
-      rest /= sp.ntiles[a];
-      origin[a] = static_cast<int>(ta * sp.tile[a]);
+      const uint32_t tiles = static_cast<uint32_t>(sp.ntiles[a]), next = rest / tiles;
+      origin[a] = static_cast<int>(rest - next * tiles) * sp.tile[a];
+      rest = next;
       const int64_t last = min(static_cast<int64_t>(origin[a]) + sp.tile[a], sp.grid.fine[a]) - 1;
       bin_lo[a] = origin[a] >> sp.grid.axis[a].shift;
       bin_hi[a] = static_cast<int>(last >> sp.grid.axis[a].shift);
@@ -957,15 +1054,12 @@ __device__ __forceinline__ void spread_part(
   }
   __syncthreads();
   const uint32_t tile_total = row_prefix[rows];
-  const uint32_t part_cap = static_cast<uint32_t>(part_cap_of(sp));
   const uint32_t record_begin = part_in_tile * part_cap;
   const uint32_t record_end = min(tile_total, record_begin + part_cap);
   // Runs of records with one support start add up in registers first (a
   // fixed order within the run) and reach the fixed-point tile once per run,
   // which leaves that much headroom in the scale.
   constexpr int kRun = spread_run<D, W, T>();
-  constexpr bool kStripCapable = strip_capable<D, W, T>();
-  constexpr bool kStrip64 = kStripCapable && sizeof(Real) == 8;
   // 2D f32: bin rows whose windows reach at most 8 rows of cells take the products.
   constexpr bool kRowCapable = row_capable<D, W, T>();
   // The order and the staged records, after the tile (spread_aux_bytes).
@@ -981,7 +1075,7 @@ __device__ __forceinline__ void spread_part(
                         2 * tile_total >= static_cast<uint32_t>(tile_cells);
   // (A warp's register sums hold at most 2^11 records of magnitude below
   // 2^27: below 2^38, which add_split takes.)
-  int S = T::exponent(max_bits[b]) - (row_path ? 3 : (kRun > 1 ? kRunBits : 0));
+  int S = T::exponent(scale_bits) - (row_path ? 3 : (kRun > 1 ? kRunBits : 0));
   const Real scale_lo = T::power_of_two(S / 2);
   const Real scale_hi = T::power_of_two(S - S / 2);
   const typename T::Complex* sv = strengths + static_cast<int64_t>(b) * point_count;
@@ -1002,7 +1096,7 @@ __device__ __forceinline__ void spread_part(
     if (strip_path) {
       // A warp's register sums hold at most 2^8 + 2^6 records of magnitude
       // below 2^29: below 2^38, which add_split takes.
-      S = T::exponent(max_bits[b]) - 1;
+      S = T::exponent(scale_bits) - 1;
       pitch0 = sp.strip_pitch0;
       pitch01 = sp.strip_pitch01;
       span = pitch01 * sp.pad[2];
@@ -1019,23 +1113,22 @@ __device__ __forceinline__ void spread_part(
     if (warp_path && !strip_path) {
       spread_warp3<W>(sp, static_cast<const PreparedWindow<3>*>(windows), sv, perm, row_begin, row_prefix, rows,
                       origin, record_begin, record_end, bucket, acc, span, sorted,
-                      reinterpret_cast<float(*)[kWarpGroup][kStageStride]>(stage), T::exponent(max_bits[b]), S);
+                      reinterpret_cast<float(*)[kWarpGroup][kStageStride]>(stage), T::exponent(scale_bits), S);
     }
   }
   if constexpr (kStrip64) {
-    // The window's Horner table in shared memory: per row the even taps, then the odd ones.
-    using L = Strip64<W>;
-    __shared__ __align__(16) double table[L::kRows * 2 * L::kTaps];
-    for (int i = tid; i < L::kRows * 2 * L::kTaps; i += kSpreadThreads) {
-      const int tap = 2 * (i % L::kTaps) + (i / L::kTaps) % 2;
-      const int r = i / (2 * L::kTaps) - (L::kRows - sp.grid.horner_rows);  // leading rows may be missing: zero
-      table[i] = tap < W && r >= 0 ? sp.grid.horner[r * W + tap] : 0.0;
-    }
-    strip_path = true;
-    spread_strips2_f64<W>(sp, reinterpret_cast<const double2*>(points), reinterpret_cast<const double2*>(sv), perm,
+    strip_path = tile_total * static_cast<uint32_t>(kStrip64CellsPerRecord) >= static_cast<uint32_t>(tile_cells);
+    if (strip_path) {
+      spread_strips2_f64<W>(sp, reinterpret_cast<const double2*>(points), reinterpret_cast<const double2*>(sv), perm,
+                            row_begin, row_prefix, rows, origin, record_begin, record_end,
+                            reinterpret_cast<unsigned long long*>(acc), padded,
+                            StripShared{sorted, strip_start, strip_cell, stage}, table, scale_lo, scale_hi);
+    } else {
+      spread_warp2_f64<W>(sp, reinterpret_cast<const double*>(points), reinterpret_cast<const double2*>(sv), perm,
                           row_begin, row_prefix, rows, origin, record_begin, record_end,
                           reinterpret_cast<unsigned long long*>(acc), padded,
-                          StripShared{sorted, strip_start, strip_cell, stage}, table, scale_lo, scale_hi);
+                          reinterpret_cast<double(*)[2][W]>(stage), table, scale_lo, scale_hi);
+    }
   }
   constexpr bool kWarp64 = D == 3 && sizeof(Real) == 8 && W > kReg64MaxWidth;
   __shared__ double stage64[kWarp64 ? kSpreadWarps : 1][kWarp64 ? D : 1][kWarp64 ? W : 1];
@@ -1206,6 +1299,8 @@ __device__ __forceinline__ void spread_part(
   // good here (kProductLoss).
   const float down_lo = T::kPreparedWindows ? ldexpf(1.0f, -S / 2) : 0.0f;
   const float down_hi = T::kPreparedWindows ? ldexpf(1.0f, -S - (-S / 2)) : 0.0f;
+  const double down64_lo = T::kPreparedWindows ? 0.0 : ldexp(1.0, -S / 2);
+  const double down64_hi = T::kPreparedWindows ? 0.0 : ldexp(1.0, -S - (-S / 2));
   auto value = [&](int which, int at) {
     if constexpr ((kStripCapable && !kStrip64) || kRowCapable) {
       if (strip_path || row_path) {
@@ -1214,7 +1309,11 @@ __device__ __forceinline__ void spread_part(
         return fmaf(hi, 65536.0f, fmaf(hi, 65536.0f * kProductLoss, lo)) * down_lo * down_hi;
       }
     }
-    return T::value(acc, span, which, at, S);
+    if constexpr (sizeof(Real) == 8) {
+      return __ll2double_rn(static_cast<long long>(acc[which * span + at])) * down64_lo * down64_hi;
+    } else {
+      return T::value(acc, span, which, at, S);
+    }
   };
   if (warp_path || (strip_path && !kStrip64)) {
     // Cells' planes and rows from reciprocals (exact: cells and pitches below 2^16).

@@ -99,8 +99,13 @@ bool spread_warp_layout(int width, const int32_t pad[3], int32_t& pitch0, int32_
 // three CTAs per SM without them.
 constexpr int kStripMinWidth = 5;
 constexpr int kStripMaxWidth = 7;
-// 2D f64 windows without register runs (spread_run) always take the strips.
+// 2D f64 windows without register runs (spread_run) take the strips in tiles of
+// at least one record per so many start cells; below, a strip's sort and flush
+// cost more than its few records' w^2 adds by whole warps (1024^2 modes,
+// uniform, us per transform of w 7, strips against warps: 1/24 point per cell
+// 360 / 299, 1/16 372 / 336, 1/8 386 with strips, 416 with warps alone).
 constexpr int kStrip64MinWidth = 5;
+constexpr int kStrip64CellsPerRecord = 10;
 constexpr int kStripMaxRecords = 2048;  // records of a part under the strips, at most
 // For tests: bytes a 2D f64 strip tile of tile0 x tile1 starts takes in shared memory.
 extern "C" int64_t b200nufft_internal_strip64_tile_bytes(int32_t width, int32_t tile0, int32_t tile1);

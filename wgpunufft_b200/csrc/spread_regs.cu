@@ -26,6 +26,7 @@
 #include "device.h"
 #include "mma.cuh"
 #include "spread.h"
+#include "strips.cuh"
 
 namespace b200nufft {
 
@@ -60,19 +61,11 @@ __global__ void __launch_bounds__(kThreads, 1) spread_regs3_kernel(
   __shared__ int64_t s_tile;
   const uint32_t part = blockIdx.x;
   if (part >= part_start[sp.tile_count]) return;
+  const uint32_t part_cap = static_cast<uint32_t>(sp.part_cap_device != nullptr ? *sp.part_cap_device : sp.part_cap);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (warp == 0) {
-    // Last tile whose first part is at or below `part`, 33-fold per step.
-    int64_t low = 0, count = sp.tile_count;
-    while (count > 1) {
-      const int64_t step = (count + 32) / 33;
-      const int64_t probe = low + (lane + 1) * step;
-      const bool below = probe < low + count && part_start[probe] <= part;
-      const int passed = __popc(__ballot_sync(0xFFFFFFFFu, below));
-      count = min(step, count - passed * step);
-      low += passed * step;
-    }
-    if (lane == 0) s_tile = low;
+    const int64_t found = part_tile(part_start, sp.tile_count, part);
+    if (lane == 0) s_tile = found;
   }
   {
     const int missing = (R::kRows - sp.grid.horner_rows) * W;  // leading rows that vanish are dropped
@@ -86,12 +79,12 @@ __global__ void __launch_bounds__(kThreads, 1) spread_regs3_kernel(
   const int64_t tile = s_tile;
   int origin[3], bin_lo[3], rows_along[3], bin_hi0 = 0;
   {
-    int64_t rest = tile;
+    uint32_t rest = static_cast<uint32_t>(tile);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      const int64_t ta = rest % sp.ntiles[a];
-      rest /= sp.ntiles[a];
-      origin[a] = static_cast<int>(ta * sp.tile[a]);
+      const uint32_t tiles = static_cast<uint32_t>(sp.ntiles[a]), next = rest / tiles;
+      origin[a] = static_cast<int>(rest - next * tiles) * sp.tile[a];
+      rest = next;
       const int64_t last = min(static_cast<int64_t>(origin[a]) + sp.tile[a], sp.grid.fine[a]) - 1;
       bin_lo[a] = origin[a] >> sp.grid.axis[a].shift;
       const int hi = static_cast<int>(last >> sp.grid.axis[a].shift);
@@ -128,7 +121,6 @@ __global__ void __launch_bounds__(kThreads, 1) spread_regs3_kernel(
     if (tid == kMaxTileRows - 1) row_prefix[kMaxTileRows] = before + warp_totals[warp];
   }
   __syncthreads();
-  const uint32_t part_cap = static_cast<uint32_t>(sp.part_cap_device != nullptr ? *sp.part_cap_device : sp.part_cap);
   const uint32_t record_begin = (part - part_start[tile]) * part_cap;
   const uint32_t record_end = min(row_prefix[kMaxTileRows], record_begin + part_cap);
   const int batches = record_end > record_begin ? static_cast<int>((record_end - record_begin + kBatch - 1) / kBatch) : 0;

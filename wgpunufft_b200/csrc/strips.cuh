@@ -29,6 +29,33 @@ constexpr int kSpreadThreads = 256;
 constexpr int kSpreadWarps = kSpreadThreads / 32;
 constexpr int kStripMax = 96;           // strips of a tile, at most
 
+// Last tile whose first part is at or below `part` (one warp). Sets of about
+// one part per tile have it near tile `part`, which costs one load's latency
+// (on every CTA's critical path); elsewhere the warp narrows the range 33-fold per
+// load.
+__device__ __forceinline__ int64_t part_tile(const uint32_t* part_start, int64_t tiles, uint32_t part) {
+  const int lane = threadIdx.x & 31;
+  int64_t low = 0, count = tiles;  // the tile lies in [low, low + count)
+  int64_t near = static_cast<int64_t>(part) - 15;
+  near = near > tiles - 32 ? tiles - 32 : near;
+  near = near < 0 ? 0 : near;
+  int64_t step = (count + 32) / 33;
+  const int64_t far = (lane + 1) * step;
+  const bool near_below = near + lane < tiles && part_start[near + lane] <= part;
+  bool below = far < tiles && part_start[far] <= part;
+  const int before = __popc(__ballot_sync(0xFFFFFFFFu, near_below));
+  if (before > 0 && (before < 32 || near + 32 >= tiles)) return near + before - 1;
+  while (count > 1) {
+    const int passed = __popc(__ballot_sync(0xFFFFFFFFu, below));
+    count = min(step, count - passed * step);
+    low += passed * step;
+    step = (count + 32) / 33;
+    const int64_t probe = low + (lane + 1) * step;
+    below = count > 1 && probe < low + count && part_start[probe] <= part;
+  }
+  return low;
+}
+
 // Shared memory of the strips beside the tile: records in strip order, first
 // record of every strip, every strip's start cell (x | y << 8 | z << 16) and
 // the warps' staged chunks.
@@ -607,6 +634,17 @@ struct Strip64 {
   static constexpr int kRows = W + 3 < kMaxHornerCoefficients ? W + 3 : kMaxHornerCoefficients;
   static constexpr int kTaps = (W + 3) / 4 * 2;
 };
+// Fills the window's Horner table: per row the even taps, then the odd ones;
+// leading rows that the fit dropped are zero. The caller synchronizes.
+template <int W>
+__device__ __forceinline__ void strip64_table(const GridParams& grid, double* table) {
+  using L = Strip64<W>;
+  for (int i = threadIdx.x; i < L::kRows * 2 * L::kTaps; i += kSpreadThreads) {
+    const int tap = 2 * (i % L::kTaps) + (i / L::kTaps) % 2;
+    const int r = i / (2 * L::kTaps) - (L::kRows - grid.horner_rows);
+    table[i] = tap < W && r >= 0 ? grid.horner[r * W + tap] : 0.0;
+  }
+}
 template <int W>
 __host__ __device__ constexpr int strip64_count(int t0, int t1) {
   return ((t0 + kStrip64X - 1) / kStrip64X) * ((t1 + Strip64<W>::S - 1) / Strip64<W>::S);
