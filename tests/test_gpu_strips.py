@@ -264,3 +264,26 @@ def test_2d_f64_sparse_and_crowded_tiles(eps, n_modes):
     want = gpu_direct.direct_type1(points, inputs, n_modes)
     for b in range(3):
         assert rel(got[b], want[b]) < max(20 * eps, 2e-13)
+
+
+@pytest.mark.parametrize("eps, tile", [(1e-6, (18, 10, 10)), (1e-9, (15, 15, 7)), (1e-11, (13, 13, 5))])
+def test_3d_f64_crowd_where_register_tiles_meet(eps, tile):
+    """All points in the bins around a corner of eight tiles, which count them all
+    and spread their own: the parts stay within those reserved."""
+    import wgpunufft_b200 as w
+
+    n_modes, count = (30, 25, 20), 200_003
+    rng = np.random.default_rng(19)
+    fine = np.asarray([2 * n for n in n_modes])
+    plan = w.NufftPlan.type1_gpu(w.NufftConfig(n_modes, eps, precision=w.Precision.F64))
+    width = plan.kernel_width()
+    assert tile == (24 - width + 1, (16 if width <= 9 else 24) - width + 1, 16 - width + 1)
+    # Support starts (cells) within 1.5 of the corner at 2 x, 1 y and 1 z tiles.
+    corner = np.asarray(tile) * (2, 1, 1)
+    x = (corner + rng.uniform(-1.5, 1.5, (count, 3)) + width / 2 - fine / 2) * 2 * np.pi / fine
+    points = np.remainder(x + np.pi, 2 * np.pi) - np.pi
+    inputs = values(rng, 2, count).astype(np.complex128)
+    _, got = transform(w, 1, n_modes, eps, w.Precision.F64, 2, points, inputs, int(np.prod(n_modes)))
+    want = gpu_direct.direct_type1(points, inputs, n_modes)
+    for b in range(2):
+        assert rel(got[b], want[b]) < max(32 * eps, 2e-13)

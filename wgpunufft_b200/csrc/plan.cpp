@@ -16,10 +16,6 @@ namespace b200nufft {
 namespace {
 
 constexpr double kTwoPi = 6.28318530717958647692;
-// Records of one spreading subproblem, at most.
-constexpr int32_t kPartCap = 4096;
-// Padded tile bytes a spreading CTA may hold, so that two fit on an SM.
-constexpr int64_t kTileBytesTarget = 100 * 1024;
 // Points one plan can bin: look-back words hold 30-bit counts.
 constexpr int64_t kMaxPoints = (int64_t(1) << 30) - 1;
 // Active batches from which 2D f32 type-2 plans stage bin regions in shared memory.
@@ -315,6 +311,9 @@ NufftPlan::NufftPlan(const b200nufft_config& c, bool with_device) : has_device_(
   check_cuda(cudaMemset(counters_.get(), 0, 8 * sizeof(uint32_t)), "clear sort tickets");
   hist_.reserve(4 * 256 * sizeof(uint32_t), "digit histograms");
   max_bits_.reserve(static_cast<size_t>(batch_) * sizeof(uint64_t), "strength maxima");
+  // Records per part, and the tiles' records (cleared by each reader for the next).
+  part_cap_.reserve(2 * sizeof(uint64_t), "part cap");
+  check_cuda(cudaMemset(part_cap_.get(), 0, 2 * sizeof(uint64_t)), "clear part cap");
 }
 
 NufftPlan::~NufftPlan() {
@@ -412,73 +411,27 @@ void NufftPlan::configure_tiles() {
   std::memset(&sp, 0, sizeof(sp));
   sp.grid = grid_;
   const int w = kernel_.width;
-  const b200nufft_tuning tuning = tuned_;
-  int64_t tile[3] = {1, 1, 1};
-  if (dim_ == 1) tile[0] = 1024;
-  // 2D f32 register runs (w <= 7) slide along the rows of 64 x 64 tiles:
-  // a thread's range of consecutive records then spans more starts of a row.
-  const bool runs2d = dim_ == 2 && precision_ == B200NUFFT_PRECISION_F32 && 2 * w * w * 4 < 400;
-  if (dim_ == 2) tile[0] = tile[1] = runs2d ? 64 : 32;
-  if (dim_ == 3) tile[0] = tile[1] = tile[2] = 16;
-  if (tuning.tile > 0) {
-    for (int a = 0; a < dim_; ++a) tile[a] = tuning.tile;
-  }
-  for (int a = 0; a < dim_; ++a) tile[a] = std::min(tile[a], pow2_ceil(fine_[a]));
-  // 3D f64 tiles spread in registers have the one shape that fills them.
-  const bool regs64 = dim_ == 3 && precision_ != B200NUFFT_PRECISION_F32 && w >= kReg64MinWidth && w <= kReg64MaxWidth;
-  if (regs64) {
-    tile[0] = kReg64Planes - w + 1;
-    tile[1] = 8 * reg64_blocks_y(w) - w + 1;
-    tile[2] = 8 * reg64_blocks_z(w) - w + 1;
-  }
-  sp.regs64 = regs64 ? 1 : 0;
-  // The tensor-core spreader needs one-cell bin rows, column bins of at most
-  // 8 cells, and its own tile shape (16 cells x 22 - w rows).
+  const bool f64 = precision_ != B200NUFFT_PRECISION_F32;
+  // The tensor-core spreader needs one-cell bin rows and column bins of at
+  // most 8 cells.
   tc_active_ = tc_enabled_ && grid_.axis[1].shift == 0 && grid_.axis[0].shift <= 3;
-  if (tc_active_) {
-    tile[0] = kTcTileX;
-    tile[1] = tc_tile_rows(w);
+  const TileShape shape = tile_shape(grid_, f64, tc_active_, tuned_, point_count_);
+  int64_t tile[3];
+  for (int a = 0; a < 3; ++a) {
+    tile[a] = shape.tile[a];
+    sp.tile[a] = shape.tile[a];
+    sp.pad[a] = shape.pad[a];
+    sp.ntiles[a] = shape.ntiles[a];
   }
-  auto padded_bytes = [&]() {
-    int64_t cells = 1;
-    for (int a = 0; a < dim_; ++a) cells *= tile[a] + w - 1;
-    return cells * 16;
-  };
-  while (!tc_active_ && !regs64 && padded_bytes() > kTileBytesTarget) {
-    int largest = dim_ - 1;
-    for (int a = dim_ - 1; a >= 0; --a) {
-      if (tile[a] > tile[largest]) largest = a;
-    }
-    if (tile[largest] == 1) break;
-    tile[largest] /= 2;
-  }
-  sp.tile_count = 1;
-  sp.padded_cells = 1;
-  int64_t tiles_per_bin = 1;
-  int64_t rows = 1;
-  for (int a = 0; a < dim_; ++a) {
-    sp.tile[a] = static_cast<int32_t>(tile[a]);
-    sp.pad[a] = static_cast<int32_t>(tile[a] + w - 1);
-    sp.ntiles[a] = static_cast<int32_t>((fine_[a] + tile[a] - 1) / tile[a]);
-    sp.tile_count *= sp.ntiles[a];
-    sp.padded_cells *= sp.pad[a];
-    const int64_t side = int64_t(1) << grid_.axis[a].shift;
-    // Tiles that a bin can meet, and bins that a tile can: tiles of no whole
-    // number of bins (or bins of no whole number of tiles) share some.
-    if (tile[a] % side != 0) tiles_per_bin *= side % tile[a] == 0 ? side / tile[a] : (side + tile[a] - 2) / tile[a] + 1;
-    if (a > 0) rows *= tile[a] % side == 0 ? tile[a] / side : (side % tile[a] == 0 ? 1 : (tile[a] + side - 2) / side + 1);
-  }
-  for (int a = dim_; a < 3; ++a) {
-    sp.tile[a] = 1;
-    sp.pad[a] = 1;
-    sp.ntiles[a] = 1;
-  }
-  if (rows > kMaxTileRows) {
+  sp.tile_count = shape.tile_count;
+  sp.padded_cells = shape.padded_cells;
+  sp.regs64 = shape.regs64;
+  if (shape.rows > kMaxTileRows) {
     throw NufftFailure{B200NUFFT_INTERNAL, "spreading tile spans too many bin rows"};
   }
   // 3D f32 tiles of widths 5 to 8: the shared-memory pitches and the segment
   // table of the warp spreader (uploaded when the tile shape changes).
-  if (dim_ == 3 && precision_ == B200NUFFT_PRECISION_F32 && w >= kWarpMinWidth && w <= kWarpMaxWidth) {
+  if (dim_ == 3 && !f64 && w >= kWarpMinWidth && w <= kWarpMaxWidth) {
     uint32_t table[32 * warp_max_rounds()];
     int32_t pitch0 = 0, pitch01 = 0;
     if (spread_warp_layout(w, sp.pad, pitch0, pitch01, table)) {
@@ -495,55 +448,23 @@ void NufftPlan::configure_tiles() {
       sp.warp_segments = static_cast<const uint32_t*>(warp_segments_.get());
     }
   }
-  sp.products = precision_ == B200NUFFT_PRECISION_F32 && !cuda_cores_only_ ? 1 : 0;
+  sp.products = !f64 && !cuda_cores_only_ ? 1 : 0;
   if (dim_ == 3 && sp.products != 0 && w >= kStripMinWidth && w <= kStripMaxWidth) {
     spread_strip_layout(sp.pad, sp.strip_pitch0, sp.strip_pitch01);
   }
-  // Parts of at most kPartCap records (f64), fewer for small point sets so that
-  // about four CTAs per SM have work. On one-cell bins holding eight or more
-  // points per cell, consecutive records share their start: parts sized for
-  // one CTA per SM give every thread runs several times longer, and the
-  // warps' flushes, which would otherwise all land on the same few windows,
-  // fall on more cells and come less often.
-  // (Register runs are taken in 1D, and in 2D while the 2 w^2 accumulators
-  // fit: spread_run in spread.cu.)
-  const int64_t real_bytes = precision_ == B200NUFFT_PRECISION_F32 ? 4 : 8;
-  const bool runs = dim_ == 1 || (dim_ == 2 && 2 * w * w * real_bytes < 400);
-  bool one_cell_bins = true;
-  for (int a = 0; a < dim_; ++a) one_cell_bins = one_cell_bins && grid_.axis[a].shift == 0;
-  const bool crowded = runs && one_cell_bins && point_count_ >= 8 * grid_.fine_count;
-  const int64_t spread_ctas = (crowded ? tuning.crowded_ctas_per_sm : tuning.ctas_per_sm) * int64_t{148};
-  int64_t cap = (std::max<int64_t>(point_count_, 1) + spread_ctas - 1) / spread_ctas;
-  // 3D parts stay within the 2048 records that crowded tiles bucket in shared
-  // memory; 1D and 2D f32 parts take up to 16384 records, so that a thread's
-  // register runs can reach 64 records in crowded tiles.
-  // The f64 strips order at most kStripMaxRecords records.
-  const bool strips64 = dim_ == 2 && precision_ != B200NUFFT_PRECISION_F32 && w >= kStrip64MinWidth;
-  const int64_t part_cap = dim_ == 3 || strips64 ? kStripMaxRecords
-                                                 : (precision_ == B200NUFFT_PRECISION_F32 ? 16384 : kPartCap);
-  cap = std::min<int64_t>(part_cap, std::max<int64_t>(256, (cap + 255) / 256 * 256));
-  sp.part_cap = static_cast<int32_t>(cap);
-  // The device sizes the parts from the points within reach (the others sort
-  // after every bin), so that such points change no part; the host bounds the
-  // parts for any count up to point_count_: valid / cap(valid) is at most
-  // 4 x 148, or point_count_ / part_cap once the cap saturates.
-  const int64_t most_ctas = std::max(tuning.ctas_per_sm, tuning.crowded_ctas_per_sm) * int64_t{148};
-  int64_t records_per_cap = most_ctas;
+  sp.part_cap = shape.part_cap;
   if (type_ == 1) {
-    sp.part_cap_device = static_cast<int32_t*>(part_cap_.reserve(sizeof(int32_t), "part cap"));
-    sp.cap_ctas = tuning.ctas_per_sm * 148;
-    sp.cap_ctas_crowded = tuning.crowded_ctas_per_sm * 148;
-    sp.cap_max = static_cast<int32_t>(part_cap);
-    sp.crowded_points = runs && one_cell_bins ? 8 * grid_.fine_count : std::numeric_limits<int64_t>::max();
+    // The device sizes the parts from the points within reach (the others sort
+    // after every bin), so that such points change no part.
+    sp.part_cap_device = static_cast<int32_t*>(part_cap_.get());
+    sp.cap_ctas = shape.cap_ctas;
+    sp.cap_ctas_crowded = shape.cap_ctas_crowded;
+    sp.cap_max = shape.cap_max;
+    sp.cap_parts = shape.cap_parts;
+    sp.crowded_points = shape.crowded_points;
     sp.cap_bins = bins_;
-    records_per_cap = std::max<int64_t>(most_ctas, (std::max<int64_t>(point_count_, 0) + part_cap - 1) / part_cap);
   }
-  // (A part but for a tile's last holds at least 256 records.)
-  const int64_t full_parts =
-      std::min(tiles_per_bin * records_per_cap, tiles_per_bin * std::max<int64_t>(point_count_, 0) / 256);
-  const int64_t part_bound = type_ == 1 ? sp.tile_count + full_parts + 1
-                                        : sp.tile_count + (std::max<int64_t>(point_count_, 0) * tiles_per_bin +
-                                                           sp.part_cap - 1) / sp.part_cap + 1;
+  const int64_t part_bound = shape.part_bound;
   // Candidate (tile, local) pairs of every coordinate of every axis: tile t
   // covers cells (t * tile + l) mod n for l < pad. They depend on the grid
   // and tile shape only, so later point sets reuse them.

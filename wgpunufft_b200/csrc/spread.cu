@@ -144,16 +144,27 @@ __device__ __forceinline__ int32_t part_cap_of(const SpreadParams& sp) {
   return sp.part_cap_device != nullptr ? *sp.part_cap_device : sp.part_cap;
 }
 
-// The part cap from the number of points within reach (SpreadParams).
-__global__ void part_cap_kernel(SpreadParams sp, const uint32_t* __restrict__ offsets) {
+// The part cap from the number of points within reach and, where they size the
+// parts (SpreadParams::cap_parts), from the tiles' records, whose sum is cleared
+// for the next point set. One thread.
+__device__ __forceinline__ unsigned long long* tile_records_sum(const SpreadParams& sp) {
+  return reinterpret_cast<unsigned long long*>(sp.part_cap_device) + 1;
+}
+__device__ __forceinline__ void set_part_cap(const SpreadParams& sp, const uint32_t* offsets) {
   const long long valid = offsets[sp.cap_bins];
   const long long ctas = valid >= sp.crowded_points ? sp.cap_ctas_crowded : sp.cap_ctas;
   long long cap = ((valid > 1 ? valid : 1ll) + ctas - 1) / ctas;
   cap = (cap + 255) / 256 * 256;
   cap = cap < 256 ? 256 : cap;
   cap = cap > sp.cap_max ? static_cast<long long>(sp.cap_max) : cap;
+  if (sp.cap_parts > 0) {
+    const long long least = (static_cast<long long>(*tile_records_sum(sp)) + sp.cap_parts - 1) / sp.cap_parts;
+    *tile_records_sum(sp) = 0ull;
+    cap = max(cap, (least + 255) / 256 * 256);
+  }
   *sp.part_cap_device = static_cast<int32_t>(cap);
 }
+__global__ void part_cap_kernel(SpreadParams sp, const uint32_t* __restrict__ offsets) { set_part_cap(sp, offsets); }
 
 // Largest |re| or |im| of every strength vector, as magnitude bits, over
 // the points within reach when a mask is given (others get zero weight, so
@@ -241,19 +252,68 @@ __global__ void tile_records_kernel(SpreadParams sp, const uint32_t* __restrict_
   parts[t] = static_cast<uint32_t>((count + cap - 1) / cap);
 }
 
+// Records in the reach of every tile's bins and their sum, for plans whose parts
+// they size: a warp per 3D tile, whose bin rows are many.
+__global__ void __launch_bounds__(256) tile_reach_kernel(SpreadParams sp, const uint32_t* __restrict__ offsets,
+                                                         uint32_t* __restrict__ records) {
+  __shared__ unsigned long long sum;
+  if (threadIdx.x == 0) sum = 0ull;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t t = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (t < sp.tile_count) {
+    uint32_t rest = static_cast<uint32_t>(t);
+    int lo[3], hi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t tiles = static_cast<uint32_t>(sp.ntiles[a]), next = rest / tiles;
+      const int origin = static_cast<int>(rest - next * tiles) * sp.tile[a];
+      rest = next;
+      const int64_t last = min(static_cast<int64_t>(origin) + sp.tile[a], sp.grid.fine[a]) - 1;
+      lo[a] = origin >> sp.grid.axis[a].shift;
+      hi[a] = static_cast<int>(last >> sp.grid.axis[a].shift);
+    }
+    const int ny = hi[1] - lo[1] + 1, rows = ny * (hi[2] - lo[2] + 1);
+    uint32_t count = 0;
+    for (int r = lane; r < rows; r += 32) {
+      const int z = r / ny, y = r - z * ny;
+      const uint64_t row = static_cast<uint64_t>(sp.grid.axis[0].bins) *
+                           (lo[1] + y + static_cast<uint64_t>(sp.grid.axis[1].bins) * (lo[2] + z));
+      count += offsets[row + hi[0] + 1] - offsets[row + lo[0]];
+    }
+    count = __reduce_add_sync(0xFFFFFFFFu, count);
+    if (lane == 0) {
+      records[t] = count;
+      if (count > 0) atomicAdd(&sum, static_cast<unsigned long long>(count));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && sum > 0ull) atomicAdd(tile_records_sum(sp), sum);
+}
+
 // Exclusive scan of the parts per tile in one block; part_start[tile_count]
-// receives the total.
-__global__ void __launch_bounds__(1024) part_scan_kernel(const uint32_t* __restrict__ parts,
-                                                         int64_t tile_count,
+// receives the total. kReach: `parts` holds the tiles' records, and the part cap
+// is set first.
+template <bool kReach>
+__global__ void __launch_bounds__(1024) part_scan_kernel(SpreadParams sp, const uint32_t* __restrict__ offsets,
+                                                         const uint32_t* __restrict__ parts, int64_t tile_count,
                                                          uint32_t* __restrict__ part_start) {
   __shared__ uint32_t warp_sums[32];
   __shared__ uint32_t carry_shared;
-  if (threadIdx.x == 0) carry_shared = 0;
+  __shared__ uint32_t cap_shared;
+  if (threadIdx.x == 0) {
+    carry_shared = 0;
+    if constexpr (kReach) {
+      set_part_cap(sp, offsets);
+      cap_shared = static_cast<uint32_t>(*sp.part_cap_device);
+    }
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t base = 0; base < tile_count; base += 1024) {
     const int64_t i = base + threadIdx.x;
-    const uint32_t v = i < tile_count ? parts[i] : 0u;
+    uint32_t v = i < tile_count ? parts[i] : 0u;
+    if constexpr (kReach) v = (v + cap_shared - 1) / cap_shared;
     uint32_t x = v;
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
@@ -1973,6 +2033,12 @@ size_t spread_shared_bytes(const SpreadParams& sp) {
 void spread_count_parts(const SpreadParams& sp, const uint32_t* offsets, uint32_t* parts,
                         uint32_t* part_start, cudaStream_t stream, StageTimer* timer) {
   StageScope scope(timer, kStageTileParts, stream);
+  if (sp.cap_parts > 0) {
+    tile_reach_kernel<<<static_cast<unsigned>((sp.tile_count + 7) / 8), 256, 0, stream>>>(sp, offsets, parts);
+    part_scan_kernel<true><<<1, 1024, 0, stream>>>(sp, offsets, parts, sp.tile_count, part_start);
+    note_launch(2);
+    return;
+  }
   if (sp.part_cap_device != nullptr) {
     part_cap_kernel<<<1, 1, 0, stream>>>(sp, offsets);
     note_launch();
@@ -1983,12 +2049,12 @@ void spread_count_parts(const SpreadParams& sp, const uint32_t* offsets, uint32_
     case 2: tile_records_kernel<2><<<blocks, 256, 0, stream>>>(sp, offsets, parts); break;
     default: tile_records_kernel<3><<<blocks, 256, 0, stream>>>(sp, offsets, parts); break;
   }
-  part_scan_kernel<<<1, 1024, 0, stream>>>(parts, sp.tile_count, part_start);
+  part_scan_kernel<false><<<1, 1024, 0, stream>>>(sp, offsets, parts, sp.tile_count, part_start);
   note_launch(2);
 }
 
 void exclusive_scan_u32(const uint32_t* in, int64_t n, uint32_t* out, cudaStream_t stream) {
-  part_scan_kernel<<<1, 1024, 0, stream>>>(in, n, out);
+  part_scan_kernel<false><<<1, 1024, 0, stream>>>(SpreadParams{}, nullptr, in, n, out);
   note_launch();
 }
 

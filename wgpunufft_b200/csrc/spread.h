@@ -5,6 +5,7 @@
 
 #include <cstdint>
 
+#include "b200_nufft.h"
 #include "device.h"
 
 namespace b200nufft {
@@ -28,11 +29,15 @@ struct SpreadParams {
   // on the device from the number of points within reach (offsets[cap_bins]):
   // part_cap_device receives min(cap_max, max(256, ceil(valid / ctas)
   // rounded up to 256)), ctas = cap_ctas_crowded when valid >=
-  // crowded_points, else cap_ctas; null keeps the host's part_cap.
+  // crowded_points, else cap_ctas; null keeps the host's part_cap. Where
+  // cap_parts is set, the cap also is at least the tiles' records (a record
+  // counts in every tile that its bin meets) over cap_parts, whatever cap_max;
+  // their sum is taken in the second 64-bit word behind part_cap_device.
   int32_t* part_cap_device;
   int32_t cap_ctas;
   int32_t cap_ctas_crowded;
   int32_t cap_max;
+  int64_t cap_parts;
   int64_t crowded_points;
   uint64_t cap_bins;
   // For each axis, candidate (tile, local) pairs of every coordinate:
@@ -63,6 +68,26 @@ struct SpreadParams {
   // (fold_dest_kernel), in the same order as the row fold.
   int32_t dest_fold;
 };
+
+// Tiles, parts and the largest number of parts (tile_shape, tiles.cpp).
+struct TileShape {
+  int32_t tile[3], pad[3], ntiles[3];
+  int64_t tile_count;
+  int32_t padded_cells;
+  int32_t regs64;
+  int64_t rows;  // bin rows of a tile
+  int32_t part_cap, cap_max, cap_ctas, cap_ctas_crowded;
+  int64_t cap_parts, crowded_points;
+  int64_t part_bound;
+};
+// The tiles of `points` points binned as `grid` says (dimensions, width, fine axes
+// and bin shifts).
+TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const b200nufft_tuning& tuning,
+                     int64_t points);
+// For tests: regs64, the tile's sides, tile count, padded cells, rows, part bound
+// and cap_parts under the default tuning.
+extern "C" int b200nufft_internal_tile_shape(int32_t dimensions, int32_t f64, int32_t width, const int64_t* fine,
+                                             const int64_t* bin_side, int64_t points, int64_t* out);
 
 // Window widths spread by whole warps, one record at a time (3D f32).
 constexpr int kWarpMinWidth = 5;
