@@ -287,3 +287,24 @@ def test_3d_f64_crowd_where_register_tiles_meet(eps, tile):
     want = gpu_direct.direct_type1(points, inputs, n_modes)
     for b in range(2):
         assert rel(got[b], want[b]) < max(32 * eps, 2e-13)
+
+
+@pytest.mark.parametrize("eps", [1e-4, 1e-5, 1e-6, 1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-12])  # widths 5 to 13
+def test_3d_f64_sparse_tiles_spread_in_shared_memory(eps):
+    """One point set below the density of the register tiles, one above, on one plan."""
+    import torch
+
+    import wgpunufft_b200 as w
+
+    n_modes = (40, 41, 38)
+    rng = np.random.default_rng(20)
+    plan = w.NufftPlan.type1_gpu(w.NufftConfig(n_modes, eps, batch=2, precision=w.Precision.F64))
+    out = torch.empty((2, int(np.prod(n_modes))), dtype=torch.complex128, device="cuda")
+    for count in (301, 12_001, 300):
+        points = rng.uniform(-np.pi, np.pi, (count, 3))
+        inputs = values(rng, 2, count).astype(np.complex128)
+        plan.encode_type1_gpu(torch.from_numpy(points).cuda(), torch.from_numpy(inputs).cuda(), out)
+        plan.synchronize()
+        want = gpu_direct.direct_type1(points, inputs, n_modes)
+        for b in range(2):
+            assert rel(out[b].cpu().numpy(), want[b]) < max(32 * eps, 2e-13)

@@ -55,13 +55,16 @@ def shared_memory_tiles(width, fine, points):
 def test_3d_f64_register_tiles_reserve_no_more_than_shared_memory_tiles(width):
     """Register tiles are no whole number of bins, whose records therefore count
     in up to eight tiles; the scratch is bounded by the points all the same."""
+    chosen = set()
     for fine in ((60, 50, 40), (128, 128, 128), (200, 180, 144), (400, 400, 400), (512, 512, 512)):
         for points in (2_000, 20_000, 150_000, 10**6, 10**7, 5 * 10**7, 2 * 10**8, 10**9):
             for side in ((2, 1, 1), (2, 2, 2), (2, 2, 4), (4, 4, 4), (4, 8, 8)):
                 s = tile_shape(3, 1, width, fine, side, points)
+                chosen.add(s["regs64"])
                 assert s["rows"] <= 256
                 if s["regs64"]:
                     assert s["parts"] * s["padded_cells"] * 16 <= max(1.1 * shared_memory_tiles(width, fine, points),
                                                                       144 * 2**20)
                     # Parts of at least records / cap_parts records each, but for a tile's last.
                     assert s["parts"] <= s["tiles"] + s["cap_parts"] + 1
+    assert chosen == {0, 1}, "sparse sets take the other tiles"

@@ -884,9 +884,10 @@ __host__ __device__ constexpr bool strip_capable() {
   return D == 3 && W >= kStripMinWidth && W <= kStripMaxWidth;
 }
 
-// 3D f64 tiles of windows wider than kReg64MaxWidth are spread by whole warps,
-// one record at a time: the lanes evaluate the 3w window taps (tap t on axis
-// t / w), and lane l adds the contributions of window cells
+// 3D f64 tiles that are not spread in registers (spread_regs.cu: too sparse or
+// too wide windows, of 5 taps or more) are spread by whole warps, one record at
+// a time: the lanes evaluate the 3w window taps (tap t on axis t / w), and lane l
+// adds the contributions of window cells
 // u = l + 32 q (x = u mod w, y = (u / w) mod w, z = u / w^2) straight to the
 // 64-bit fixed-point tile; the 32 lanes of an add touch 32 different cells.
 template <int W>
@@ -1190,7 +1191,7 @@ __device__ __forceinline__ void spread_part(
                           reinterpret_cast<double(*)[2][W]>(stage), table, scale_lo, scale_hi);
     }
   }
-  constexpr bool kWarp64 = D == 3 && sizeof(Real) == 8 && W > kReg64MaxWidth;
+  constexpr bool kWarp64 = D == 3 && sizeof(Real) == 8 && W >= kReg64MinWidth;
   __shared__ double stage64[kWarp64 ? kSpreadWarps : 1][kWarp64 ? D : 1][kWarp64 ? W : 1];
   if constexpr (kWarp64) {
     spread_warp3_f64<W>(sp, reinterpret_cast<const double*>(points), reinterpret_cast<const double2*>(sv), perm,
@@ -1753,20 +1754,16 @@ void fold_any(const SpreadParams& sp, int batch, const Complex* scratch, const u
 
 template <int D, int W, typename T>
 void launch_spread_width(const SpreadParams& sp, const SpreadLaunchT<T>& l, cudaStream_t stream) {
-  if constexpr (D == 3 && sizeof(typename T::Real) == 8 && W >= kReg64MinWidth && W <= kReg64MaxWidth) {
-    throw NufftFailure{B200NUFFT_INTERNAL, "3D f64 plans of this width spread in registers"};
-  } else {
-    const size_t smem = spread_tile_bytes<D, W, T>(sp) + spread_aux_bytes<D, W, T>();
-    auto kernel = spread_tiles_kernel<D, W, T>;
-    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)),
-               "spread shared memory");
-    const dim3 grid(static_cast<unsigned>(l.part_upper_bound), static_cast<unsigned>(l.batch));
-    kernel<<<grid, kSpreadThreads, smem, stream>>>(sp, l.points, l.windows, l.strengths, l.point_count, l.batch,
-                                                   l.perm, l.offsets, l.part_start, l.max_bits,
-                                                   l.scratch);
-    note_launch();
-  }
+  const size_t smem = spread_tile_bytes<D, W, T>(sp) + spread_aux_bytes<D, W, T>();
+  auto kernel = spread_tiles_kernel<D, W, T>;
+  check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(smem)),
+             "spread shared memory");
+  const dim3 grid(static_cast<unsigned>(l.part_upper_bound), static_cast<unsigned>(l.batch));
+  kernel<<<grid, kSpreadThreads, smem, stream>>>(sp, l.points, l.windows, l.strengths, l.point_count, l.batch,
+                                                 l.perm, l.offsets, l.part_start, l.max_bits,
+                                                 l.scratch);
+  note_launch();
 }
 
 template <int D, typename T>

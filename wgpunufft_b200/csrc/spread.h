@@ -60,7 +60,7 @@ struct SpreadParams {
   // padded tile under the tensor-core strips (spread_strip_layout).
   int32_t strip_pitch0;
   int32_t strip_pitch01;
-  // 3D f64 plans of widths kReg64MinWidth..kReg64MaxWidth: the tiles of spread_regs64.
+  // 3D f64 plans that spread in registers: the tiles of spread_regs64.
   int32_t regs64;
   // 3D plans of 16 x 16 x (4 k)-cell tiles whose cells' candidate lists are,
   // along every axis, ordered parts of the list of their tile's first cell
@@ -140,7 +140,8 @@ void spread_strip_layout(const int32_t pad[3], int32_t& pitch0, int32_t& pitch01
 
 // 3D f64 plans of these widths spread in registers (spread_regs.cu): padded
 // tiles of kReg64Planes x 8 by x 8 bz cells, tiles of w - 1 fewer starts per
-// axis. Wider windows would leave tiles of three starts or less along z.
+// axis, where the points are dense enough (tile_shape). Wider windows would leave
+// tiles of three starts or less along z.
 constexpr int kReg64MinWidth = 5;
 constexpr int kReg64MaxWidth = 13;
 constexpr int kReg64Planes = 24;

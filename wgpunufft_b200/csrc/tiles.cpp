@@ -21,6 +21,25 @@ int64_t pow2_ceil(int64_t v) {
   return p;
 }
 
+// Fine cells per point up to which 3D f64 plans spread in registers. Sparser
+// tiles leave a CTA per SM waiting for its few records and its write-out, where
+// two CTAs of the shared-memory kernel overlap. 256^3 cells, uniform, us per
+// transform, registers against shared memory: w 7, 1/64 point per cell 1443 / 1627,
+// 1/512 1323 / 1119; w 10, 1/192 1932 / 2654, 1/1536 1750 / 1397. (Scattered
+// points: the line is the earlier of that and a 180 x 140 x 200 grid.)
+int64_t reg64_cells_per_point(int w) {
+  switch (w) {
+    case 6: return 128;
+    case 8: return 64;
+    case 9: return 96;
+    case 10:
+    case 11: return 768;
+    case 12:
+    case 13: return 1536;
+    default: return 256;  // 5, 7
+  }
+}
+
 }  // namespace
 
 TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const b200nufft_tuning& tuning,
@@ -39,7 +58,8 @@ TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const 
     for (int a = 0; a < dim; ++a) tile[a] = tuning.tile;
   }
   for (int a = 0; a < dim; ++a) tile[a] = std::min(tile[a], pow2_ceil(grid.fine[a]));
-  const bool regs64 = dim == 3 && f64 && w >= kReg64MinWidth && w <= kReg64MaxWidth;
+  const bool regs64 = dim == 3 && f64 && w >= kReg64MinWidth && w <= kReg64MaxWidth &&
+                      points * reg64_cells_per_point(w) >= grid.fine_count;
   auto padded_bytes = [&]() {
     int64_t cells = 1;
     for (int a = 0; a < dim; ++a) cells *= tile[a] + w - 1;
