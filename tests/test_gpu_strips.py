@@ -308,3 +308,21 @@ def test_3d_f64_sparse_tiles_spread_in_shared_memory(eps):
         want = gpu_direct.direct_type1(points, inputs, n_modes)
         for b in range(2):
             assert rel(out[b].cpu().numpy(), want[b]) < max(32 * eps, 2e-13)
+
+
+@pytest.mark.parametrize("eps", [1e-5, 1e-6])  # widths 6 and 7
+@pytest.mark.parametrize("n_modes, count, spread, batch", [
+    ((32, 32, 32), 262_144, "uniform", 1),
+    ((21, 19, 33), 250_001, "crowded", 3),
+    ((8, 40, 13), 250_003, "edges", 2),
+])
+def test_f32_3d_values_of_many_points_differ_from_f64_by_rounding(eps, n_modes, count, spread, batch):
+    """Point sets large enough for the strips (interp_strips_chosen), in both precisions."""
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(21)
+    points = points_of(rng, spread, count, [2 * n for n in n_modes])
+    inputs = values(rng, batch, int(np.prod(n_modes)))
+    _, got = transform(w, 2, n_modes, eps, w.Precision.F32, batch, points, inputs, count)
+    _, want = transform(w, 2, n_modes, eps, w.Precision.F64, batch, points, inputs, count)
+    assert rel(got, want) < (32 * eps if spread == "edges" else F32_ROUNDING + 0.2 * eps)

@@ -428,11 +428,17 @@ void launch_width(const GridParams& g, const typename T::Real* points, const voi
 }  // namespace
 
 bool interp_strips_chosen(int dimensions, bool f64, int width, int64_t points, int64_t cells) {
-  if (f64) {
-    if (width < 5) return false;
-    return dimensions == 2 || (dimensions == 3 && points * (width < 12 ? 6 : 12) >= cells);
-  }
-  return dimensions == 3 && ((width == 6 && points * 3 >= cells) || (width == 7 && points * 4 >= cells));
+  // 2D f64 warps choose for themselves (kMostGroups).
+  if (f64 && (dimensions == 2 || width < 5)) return dimensions == 2 && width >= 5;
+  if (dimensions != 3) return false;
+  // Cells per point up to which a group's products cost less than its gathers;
+  // and points from which the warps, whose groups follow one another, are enough
+  // to hide it (20^3 to 40 x 36 x 30 modes, us per transform, gather against strips:
+  // f32 w 6, 64 000 points 29 / 33, 172 800 51 / 56, 691 200 95 / 89 (clustered, 262 000
+  // 44 / 35); w 7, 65 500 36 / 48, 87 400 47 / 43; f64 w 6, 57 600 58 / 70, 87 400 72 / 65).
+  if (f64) return points * (width < 12 ? 6 : 12) >= cells && (width > 6 || points >= 80'000);
+  return (width == 6 && points * 3 >= cells && points >= 250'000) ||
+         (width == 7 && points * 4 >= cells && points >= 80'000);
 }
 
 void interp_strip_shifts(bool f64, int32_t shift[3]) {
