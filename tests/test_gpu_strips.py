@@ -326,3 +326,27 @@ def test_f32_3d_values_of_many_points_differ_from_f64_by_rounding(eps, n_modes, 
     _, got = transform(w, 2, n_modes, eps, w.Precision.F32, batch, points, inputs, count)
     _, want = transform(w, 2, n_modes, eps, w.Precision.F64, batch, points, inputs, count)
     assert rel(got, want) < (32 * eps if spread == "edges" else F32_ROUNDING + 0.2 * eps)
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-3, 1e-4, 1e-6])  # widths 2, 4, 5, 7
+@pytest.mark.parametrize("capacity, active", [(16, 16), (20, 5), (48, 18), (48, 48)])
+@pytest.mark.parametrize("n_modes, count", [((64, 64), 2_000), ((64, 64), 33_000), ((300, 200), 9_000)])
+def test_batched_2d_type2_of_either_kernel_matches_the_bins(eps, capacity, active, n_modes, count):
+    """16 to 63 vectors, point sets on both sides of the rule: against the CUDA-core kernels."""
+    import torch
+
+    import wgpunufft_b200 as w
+
+    rng = np.random.default_rng(22)
+    points = torch.from_numpy(points_of(rng, "uniform", count, [2 * n for n in n_modes])).cuda()
+    inputs = torch.from_numpy(values(rng, active, int(np.prod(n_modes)))).cuda()
+
+    def run(method):
+        plan = w.NufftPlan.type2_gpu(w.NufftConfig(n_modes, eps, batch=capacity, spread_method=method))
+        plan.set_points_gpu(points)
+        out = torch.empty((active, count), dtype=torch.complex64, device="cuda")
+        plan.execute_type2_gpu_batch(active, inputs, out)
+        plan.synchronize()
+        return out.cpu().numpy()
+
+    assert rel(run(w.SpreadMethod.AUTO), run(w.SpreadMethod.CUDA_CORES)) < F32_ROUNDING

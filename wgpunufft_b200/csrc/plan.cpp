@@ -614,7 +614,8 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
   const size_t sorted_bytes = static_cast<size_t>(std::max<int64_t>(count, 1)) * dim_ * scalar_bytes();
   if (precision_ == B200NUFFT_PRECISION_F32) {
     tc2_active_ = tc2_enabled_ && batch_ >= kTi2Vectors && tc_interp_supported(grid_);
-    tc2_strips_ = tc2_enabled_ && !tc2_active_;
+    // (Fewer active vectors than the plan holds take the strips where they are kept.)
+    tc2_strips_ = tc2_enabled_ && !tc2_active_ && strips_for_batch(static_cast<int>(batch_));
     if (tc2_active_ && count > 0) {
       // The tensor-core order first (its permutation is consumed at once),
       // then the reference's type-2 bins in the same sort buffers.
@@ -1251,12 +1252,21 @@ bool NufftPlan::interp_strips() const {
 }
 
 bool NufftPlan::strips_for_batch(int batch) const {
-  // 2D 512^2 modes, 2e6 points, us per execution, per-bin regions of 32 vectors
-  // against strips: w 7, 16 vectors 1682 / 692, 32 vectors 1893 / 1369; w 4, 16
-  // vectors 919 / 648, 32 vectors 1056 / 1279. The tcgen05 kernel serves 64
+  // us per transform, per-bin regions of 32 vectors against strips. 512^2 modes,
+  // 2e6 points: w 7, 16 vectors 1682 / 692, 32 vectors 1893 / 1369; w 4, 16 vectors 919
+  // / 648, 32 vectors 1056 / 1279: below w 6 the regions, which serve 32 vectors for
+  // the price of 16, win from about 24 on. Few points are too few warps for the
+  // strips, whose groups follow one another, and few vectors do not fill the
+  // regions: 128^2 modes, w 7, 1640 points, 16 vectors 43 / 58, 63 vectors 100 / 78;
+  // w 5, 16 vectors, 4100 points 37 / 43, 16 400 points 41 / 39; 300^2 modes, 9000
+  // points 147 / 133; 64^2 modes, 16 400 points 30 / 21. The tcgen05 kernel serves 64
   // vectors for the price of 16 (w 7, 64 vectors: 2484 against 2727).
   if (tc_min_batch_ == 1) return true;
-  return batch >= tc_min_batch_ && kernel_.width >= 3 && (kernel_.width >= 6 || batch <= 24);
+  if (batch < tc_min_batch_ || kernel_.width < 3) return false;
+  if (kernel_.width >= 6) return point_count_ >= 3'000 || batch > 32;
+  if (batch > 24) return false;
+  if (2 * point_count_ >= fine_count_ && point_count_ >= 3'000) return true;
+  return fine_count_ >= 150'000 ? point_count_ >= 8'000 : batch <= 16 && point_count_ >= 16'000;
 }
 
 bool NufftPlan::interp_rows_order() const { return type_ == 2 && (dim_ == 3 || interp_strips()); }
