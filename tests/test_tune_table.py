@@ -58,3 +58,45 @@ def test_tensor_thresholds_merge_per_type_and_width(monkeypatch, tmp_path):
     path = tmp_path / "tuning_table.h"
     path.write_text(tune.table_header(entries))
     assert tune.read_table(path) == entries
+
+
+def test_type2_thresholds_are_measured_on_plans_that_take_them(monkeypatch):
+    """Type-2 plans below 64 vectors have no tcgen05 kernel: the threshold of
+    smaller batches is that of active vectors of a 64-vector plan."""
+    from types import SimpleNamespace
+
+    made = []
+
+    class Plan:
+        def __init__(self, kind, config):
+            self.made = [kind, config["batch"], config["spread_method"], None]
+            made.append(self.made)
+
+        def kernel_width(self):
+            return 7
+
+        def set_points_gpu(self, points):
+            pass
+
+        def execute_gpu_batch(self, active, inputs, out):
+            self.made[3] = active
+
+    w = SimpleNamespace(
+        NufftPlan=SimpleNamespace(type1_gpu=lambda c: Plan(1, c), type2_gpu=lambda c: Plan(2, c)),
+        NufftConfig=lambda modes, eps, **kw: kw,
+        SpreadMethod=SimpleNamespace(TENSOR_CORES="tensor", CUDA_CORES="cuda"))
+    torch = SimpleNamespace(empty=lambda *a, **k: None, complex64=None, cuda=SimpleNamespace(empty_cache=lambda: None))
+    workloads = SimpleNamespace(points=lambda *a, **k: None, values=lambda *a, **k: None)
+
+    def fake_time(torch, fn, repeats):
+        fn()
+        return 2.0  # no method is ever faster: every batch is measured
+
+    monkeypatch.setattr(tune, "_time", fake_time)
+    for kind in (1, 2):
+        made.clear()
+        threshold, width, _ = tune.tune_tensor_threshold(torch, w, workloads, None, kind, 1e-6, 1)
+        assert (threshold, width) == (0, 7)
+        assert [m[3] for m in made] == [b for b in tune.TENSOR_BATCHES for _ in (0, 1)]
+        for k, capacity, _, active in made:
+            assert k == kind and capacity == (active if kind == 1 else max(active, 64))

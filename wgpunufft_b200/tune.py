@@ -107,6 +107,9 @@ def tune_workload(torch, w, workloads, native, spec, repeats):
 TENSOR_MODES, TENSOR_POINTS = (512, 512), 2_000_000
 TENSOR_EPS = (1e-2, 1e-3, 1e-4, 1e-5, 1e-6)
 TENSOR_BATCHES = (16, 32, 64, 128, 256)
+# Type-2 plans of fewer vectors interpolate by strips on the tensor cores, to
+# which the thresholds do not apply: fewer are active vectors of such a plan.
+TYPE2_CAPACITY = 64
 
 
 def tune_tensor_threshold(torch, w, workloads, native, kind, eps, repeats):
@@ -124,7 +127,8 @@ def tune_tensor_threshold(torch, w, workloads, native, kind, eps, repeats):
         ms = {}
         for method in (w.SpreadMethod.TENSOR_CORES, w.SpreadMethod.CUDA_CORES):
             plan = (w.NufftPlan.type1_gpu if kind == 1 else w.NufftPlan.type2_gpu)(
-                w.NufftConfig(modes, eps, batch=batch, spread_method=method))
+                w.NufftConfig(modes, eps, batch=batch if kind == 1 else max(batch, TYPE2_CAPACITY),
+                              spread_method=method))
             width = plan.kernel_width()
             plan.set_points_gpu(pts)
             ms[method] = _time(torch, lambda: plan.execute_gpu_batch(batch, inputs, out), repeats)
