@@ -372,7 +372,10 @@ int b200nufft_batch_execute(b200nufft_batch batch, const void *const *strengths,
  * (wgpunufft_b200/tune.py) holds them per workload key: plan type,
  * dimension, precision, window width, log2 of the fine-grid cells and log2
  * of the points per cell. Plans look the key up at set_points, so a key
- * always gets the same choices and outputs stay bitwise repeatable. */
+ * always gets the same choices and outputs stay bitwise repeatable. The
+ * tensor-core batches of the table are those of type-1 plans and of type-2 plans
+ * of 64 vectors or more; type-2 plans of 16 to 63 choose by width, points and
+ * grid, unless an override sets tensor_min_batch. */
 typedef struct b200nufft_tuning {
   int32_t tile;                /* spreading tile side in cells (power of two) */
   int32_t ctas_per_sm;         /* CTAs per SM the tile parts are sized for */

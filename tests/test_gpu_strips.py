@@ -350,3 +350,36 @@ def test_batched_2d_type2_of_either_kernel_matches_the_bins(eps, capacity, activ
         return out.cpu().numpy()
 
     assert rel(run(w.SpreadMethod.AUTO), run(w.SpreadMethod.CUDA_CORES)) < F32_ROUNDING
+
+
+def test_override_sets_the_batch_of_type2_strips():
+    """tensor_min_batch of an override decides for 16 to 63 vectors too: the
+    same bits as the plan that is asked for the kernel."""
+    import torch
+
+    import wgpunufft_b200 as w
+    from wgpunufft_b200 import _native
+
+    n_modes, count, batch = (64, 64), 30_000, 32  # eps 1e-3: bins by the rule
+    rng = np.random.default_rng(23)
+    points = torch.from_numpy(points_of(rng, "uniform", count, [128, 128])).cuda()
+    inputs = torch.from_numpy(values(rng, batch, 64 * 64)).cuda()
+    override = _native.library().b200nufft_tuning_override
+
+    def run(method, least=0):
+        if least:
+            override(_native.Tuning(0, 0, 0, least))
+        try:
+            plan = w.NufftPlan.type2_gpu(w.NufftConfig(n_modes, 1e-3, batch=batch, spread_method=method))
+            out = torch.empty((batch, count), dtype=torch.complex64, device="cuda")
+            plan.encode_type2_gpu(points, inputs, out)
+            plan.synchronize()
+        finally:
+            override(None)
+        return out.view(torch.int32)
+
+    strips, bins = run(w.SpreadMethod.TENSOR_CORES), run(w.SpreadMethod.CUDA_CORES)
+    assert not torch.equal(strips, bins)
+    assert torch.equal(run(w.SpreadMethod.AUTO), bins)
+    assert torch.equal(run(w.SpreadMethod.AUTO, 16), strips)
+    assert torch.equal(run(w.SpreadMethod.AUTO, 33), bins)

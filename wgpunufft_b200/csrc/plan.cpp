@@ -570,6 +570,7 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
   point_count_ = count;
   points_ = points;
   tuned_ = tuning_for(tuning_key(type_, dim_, precision_, kernel_.width, fine_count_, count));
+  strips_min_batch_ = tensor_min_batch_override();
   if (dim_ > 3) {
     // No bins: the coordinates are kept (in f64 for Df64 plans) as given.
     const size_t coords = static_cast<size_t>(std::max<int64_t>(count, 1)) * dim_;
@@ -1262,6 +1263,7 @@ bool NufftPlan::strips_for_batch(int batch) const {
   // points 147 / 133; 64^2 modes, 16 400 points 30 / 21. The tcgen05 kernel serves 64
   // vectors for the price of 16 (w 7, 64 vectors: 2484 against 2727).
   if (tc_min_batch_ == 1) return true;
+  if (strips_min_batch_ > 0) return batch >= std::max<int64_t>(tc_min_batch_, strips_min_batch_);
   if (batch < tc_min_batch_ || kernel_.width < 3) return false;
   if (kernel_.width >= 6) return point_count_ >= 3'000 || batch > 32;
   if (batch > 24) return false;

@@ -215,6 +215,7 @@ class NufftPlan {
   // Fewer vectors: the points' strip order (interp_strips.cu) and their
   // windows in it.
   bool tc2_strips_ = false;
+  int32_t strips_min_batch_ = 0;  // an override's smallest batch for them; 0: strips_for_batch's rule
   bool strips_for_batch(int batch) const;
   DeviceBuffer tc2_perm_, tc2_windows_;
 };

@@ -77,6 +77,11 @@ b200nufft_tuning tuning_for(const TuningKey& key) {
   return t;
 }
 
+int32_t tensor_min_batch_override() {
+  std::lock_guard<std::mutex> lock(g_override_mutex);
+  return g_override_set ? g_override.tensor_min_batch : 0;
+}
+
 bool fused_fft_enabled() { return b200nufft::g_fused_transforms.load(); }
 
 }  // namespace b200nufft

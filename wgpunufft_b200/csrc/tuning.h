@@ -32,6 +32,9 @@ TuningKey tuning_key(int type, int dimensions, int precision, int width, int64_t
 // override is set. Zero fields of an override keep the table's choice.
 b200nufft_tuning tuning_for(const TuningKey& key);
 
+// The override's smallest tensor-core batch; 0 without one.
+int32_t tensor_min_batch_override();
+
 // Defaults of every field (tile 0: the plan's own default tile).
 b200nufft_tuning default_tuning(int dimensions);
 
