@@ -100,3 +100,10 @@ def test_type2_thresholds_are_measured_on_plans_that_take_them(monkeypatch):
         assert [m[3] for m in made] == [b for b in tune.TENSOR_BATCHES for _ in (0, 1)]
         for k, capacity, _, active in made:
             assert k == kind and capacity == (active if kind == 1 else max(active, 64))
+
+
+def test_committed_table_is_written_from_the_committed_measurements():
+    import json
+
+    measured = json.loads((TABLE.parents[1] / "tuning" / "tensor_thresholds_b200.json").read_text())["entries"]
+    assert tune.table_header(measured) == TABLE.read_text()

@@ -21,7 +21,7 @@ constexpr TuningEntry kTuningTable[] = {
     {1, 3, 3, 6, 27, -2, 16, 2, 1, 16},  // 3d_256_5e7_radial: 13.7454 ms
     {1, 3, 3, 7, 21, -2, 16, 4, 1, 16},  // 3d_64_1e6_uniform: 0.5508 ms
     {1, 3, 3, 7, 18, -2, 8, 2, 1, 16},  // 3d_32_1e5_clustered: 0.0966 ms
-    {1, 2, 1, 10, 20, 0, 32, 4, 1, 16},  // 2d_512_2e6_f64_1e-9: 0.5040 ms
+    {1, 2, 1, 10, 20, 0, 32, 4, 1, 16},  // 2d_512_2e6_f64_1e-9: 0.4353 ms
     {2, 2, 3, 7, 20, 0, 32, 4, 1, 64},  // 2d_512_2e6_uniform_type2: 0.1855 ms
     {1, 2, 3, 4, 20, 0, 0, 4, 1, 16},  // 2d_512_2e6_uniform_eps0.001_type1_cuda_cores_B16: 1.2732 ms
     {2, 2, 3, 4, 20, 0, 0, 4, 1, 128},  // 2d_512_2e6_uniform_eps0.001_type2_cuda_cores_B16: 1.0525 ms
