@@ -1054,12 +1054,15 @@ __device__ __forceinline__ void spread_part(
   // Tile origin and bin rows.
   int origin[3], bin_lo[3], bin_hi[3], rows_along[3];
   {
-    uint32_t rest = static_cast<uint32_t>(tile);  // parts and tiles count in 32 bits
+    // Tiles count in 32 bits; but the f32 register runs came out of the compiler
+    // slower by 16 us with it (1024^2 modes, 1e7 points, w 6: 401 -> 417).
+    using Index = std::conditional_t<sizeof(Real) == 8, uint32_t, int64_t>;
+    Index rest = static_cast<Index>(tile);
 #pragma unroll
     for (int a = 0; a < D; ++a) {
-      const uint32_t tiles = static_cast<uint32_t>(sp.ntiles[a]), next = rest / tiles;
-      origin[a] = static_cast<int>(rest - next * tiles) * sp.tile[a];
-      rest = next;
+      const Index ta = rest % static_cast<Index>(sp.ntiles[a]);
+      rest /= static_cast<Index>(sp.ntiles[a]);
+      origin[a] = static_cast<int>(ta * static_cast<Index>(sp.tile[a]));
       const int64_t last = min(static_cast<int64_t>(origin[a]) + sp.tile[a], sp.grid.fine[a]) - 1;
       bin_lo[a] = origin[a] >> sp.grid.axis[a].shift;
       bin_hi[a] = static_cast<int>(last >> sp.grid.axis[a].shift);
