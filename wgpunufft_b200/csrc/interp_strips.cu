@@ -69,8 +69,7 @@ struct F64Strips {
 // that each lane gathers its own w^2 cells, adding them in the products' order
 // (the same bits). A group's products cost a half (w 5) to a fifth (w 13) of 32
 // gathers. 1024^2 modes, uniform, us per transform with products alone and so: w 7,
-// 1/16 point per cell 195 / 139, 1/4 244 / 224, one point 392 / 401; w 13, 1/16
-// 249 / 221, one point 614 / 626.
+// 1/16 point per cell 195 / 139, 1/4 244 / 224; w 13, 1/16 249 / 221.
 template <int W>
 constexpr int kMostGroups = W <= 6 ? 1 : (W <= 8 ? 2 : (W - 1) / 2);
 
@@ -111,13 +110,14 @@ __device__ __noinline__ void gather_columns(const double* wx, const double* wy, 
   }
 }
 
-// CTAs of an SM that the registers are held to (2D f64: what the products alone
-// take, so that the gathers do not cost them their occupancy; 0: free).
-template <int D, int W, typename T>
-constexpr int kMinBlocks = D == 2 && sizeof(typename T::Real) == 8 ? (W <= 9 ? 10 : 8) : 0;
+// CTAs of an SM that the registers of a kernel with gathers are held to: what the
+// products alone take (0: free).
+template <int W, bool Scattered>
+constexpr int kMinBlocks = Scattered ? (W <= 9 ? 10 : 8) : 0;
 
-template <int D, int W, int V, typename T>
-__global__ void __launch_bounds__(T::kWarps * 32, (kMinBlocks<D, W, T>)) interp_strips_kernel(
+// Scattered: with the gathers (2D f64).
+template <int D, int W, int V, typename T, bool Scattered = false>
+__global__ void __launch_bounds__(T::kWarps * 32, (kMinBlocks<W, Scattered>)) interp_strips_kernel(
     GridParams grid, const typename T::Real* __restrict__ points, const void* __restrict__ windows, int64_t count,
     const uint32_t* __restrict__ perm, const typename T::Complex* __restrict__ fine, int batch,
     typename T::Complex* __restrict__ output) {
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(T::kWarps * 32, (kMinBlocks<D, W, T>)) interp_
     q.members = __ballot_sync(0xFFFFFFFFu, q.mine);
     return q;
   };
-  if constexpr (F64 && D == 2) {
+  if constexpr (Scattered) {
     // Points too far apart for products: every lane gathers its own.
     int groups = 0;
     for (unsigned left = todo; left != 0u && groups <= kMostGroups<W>; ++groups) left &= ~next_group(left).members;
@@ -416,6 +416,17 @@ void launch_width(const GridParams& g, const typename T::Real* points, const voi
     if (batch > 1) {
       interp_strips_kernel<D, W, kBlockVectors, T><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count,
                                                                                           perm, fine, batch, output);
+      note_launch();
+      return;
+    }
+  }
+  if constexpr (D == 2 && sizeof(typename T::Real) == 8) {
+    // From half a point per cell on (w 11 and wider: a twelfth) few warps are
+    // scattered, and the kernel without gathers, whose bits are the same, is 1 to
+    // 4 % faster.
+    if ((W <= 10 ? 2 : 12) * count < g.fine_count) {
+      interp_strips_kernel<D, W, 1, T, true><<<blocks, T::kWarps * 32, 0, stream>>>(g, points, windows, count, perm,
+                                                                                    fine, batch, output);
       note_launch();
       return;
     }
