@@ -383,3 +383,27 @@ def test_override_sets_the_batch_of_type2_strips():
     assert torch.equal(run(w.SpreadMethod.AUTO), bins)
     assert torch.equal(run(w.SpreadMethod.AUTO, 16), strips)
     assert torch.equal(run(w.SpreadMethod.AUTO, 33), bins)
+
+
+@pytest.mark.parametrize("kind", [1, 2])
+@pytest.mark.parametrize("n_modes, count", [((33, 21), 9_001), ((14, 11, 13), 12_001)])
+@pytest.mark.parametrize("width", range(5, 17))
+def test_f64_vectors_of_a_batch_are_those_of_single_calls(kind, n_modes, count, width):
+    """Every width's kernels, five vectors: each the bits of a call of its own,
+    the last one the direct sums."""
+    import wgpunufft_b200 as w
+
+    eps = 10.0 ** (1 - width)
+    rng = np.random.default_rng(24)
+    points = points_of(rng, "crowded", count, [2 * n for n in n_modes]).astype(np.float64)
+    total = int(np.prod(n_modes))
+    inputs = values(rng, 5, count if kind == 1 else total).astype(np.complex128)
+    outputs = total if kind == 1 else count
+    plan, got = transform(w, kind, n_modes, eps, w.Precision.F64, 5, points, inputs, outputs)
+    assert plan.kernel_width() == width
+    for b in (0, 4):
+        _, alone = transform(w, kind, n_modes, eps, w.Precision.F64, 1, points, inputs[b : b + 1], outputs)
+        assert np.array_equal(got[b].view(np.float64), alone[0].view(np.float64))
+    direct = gpu_direct.direct_type1 if kind == 1 else gpu_direct.direct_type2
+    want = direct(points, inputs[4:5], n_modes)[0]
+    assert rel(got[4], want) < max((20 if len(n_modes) == 2 else 32) * eps, 2e-13)
