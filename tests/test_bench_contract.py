@@ -43,3 +43,24 @@ def test_reference_arm_other_ranks_exit_quietly():
     done = run_reference_arm({"RANK": "1"})
     assert done.returncode == 0, done.stderr[-2000:]
     assert not [line for line in done.stdout.splitlines() if line.startswith("{")]
+
+
+def test_the_json_line_is_short_and_whole():
+    """A reader that keeps the last 3,000 characters of the output gets the whole line."""
+    sys.path.insert(0, str(ROOT))
+    import bench
+
+    number, text = 12345678901.234567, "x" * 300
+    line = {k: number for k in bench.LINE_KEYS}
+    line.update(metric=bench.METRIC, data=text[:60], config={k: text[:60] for k in "abcdefgh"},
+                e2e={"value": number, "unit": "points/s", "ms_per_step": number, "h2d_bytes_per_step": 160000000,
+                     "d2h_bytes_per_step": 8388608, "path": text},
+                clocks={"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": [], "samples": 2},
+                roofline={**{k: number for k in "abcdefg"}, "traffic_source": text, "peak_source": text[:60]},
+                cpu_baseline={"value": number, "sample": text, "one_shot_value": number})
+    line.update(batched={"entries": [text] * 100}, type2={"value": number, "rel_l2": 1e-5, "stages": text},
+                one_shot={"value": number}, summary={"all": text})
+    details, short = bench.split_line(line)
+    assert len(json.dumps(short, separators=(",", ":"))) < 2_900
+    assert set(bench.LINE_KEYS) <= set(short) and short["type2"]["value"] > 0
+    assert set(details) | set(short) >= set(line) and "batched" in details
