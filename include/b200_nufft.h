@@ -212,9 +212,9 @@ int b200nufft_encode(b200nufft_plan plan, int64_t active_batch, int64_t point_co
  * every slot and `bin_offsets` (device, bin_count + 1 words) the first slot of
  * every bin followed by the total (NdPointBins::encode,
  * src/gpu_nd_bins.rs:336-471). Either pointer may be null. 3D type-2
- * plans, and 2D f64 ones of eps below 1e-3, interpolate in another order and
- * sort the bin order at the first call after each set_points, on `stream` (3D
- * plans reserve a device buffer of 3 coordinates per point the first time). */
+ * plans, and 2D f64 ones of a window of 5 points or more (eps below 1e-3 at sigma
+ * 2), interpolate in another order and sort the bin order at the first call
+ * after each set_points, on `stream` (3D plans reserve a device buffer of 3 coordinates per point the first time). */
 int b200nufft_copy_bin_order(b200nufft_plan plan, uint32_t *permutation,
                              uint32_t *bin_offsets, void *stream);
 
