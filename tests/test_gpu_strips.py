@@ -407,3 +407,48 @@ def test_f64_vectors_of_a_batch_are_those_of_single_calls(kind, n_modes, count, 
     direct = gpu_direct.direct_type1 if kind == 1 else gpu_direct.direct_type2
     want = direct(points, inputs[4:5], n_modes)[0]
     assert rel(got[4], want) < max((20 if len(n_modes) == 2 else 32) * eps, 2e-13)
+
+
+@pytest.mark.parametrize("kind, n_modes, eps, precision, batch, many, few", [
+    (1, (48, 40, 44), 1e-9, "F64", 2, 60_000, 500),     # register tiles; shared-memory tiles
+    (2, (48, 40, 44), 1e-9, "F64", 1, 200_000, 3_000),  # strips; the gather's order
+    (2, (48, 40, 44), 1e-6, "F32", 1, 400_000, 5_000),
+    (2, (100, 90), 1e-6, "F32", 16, 60_000, 2_000),     # strips; bins
+    (2, (100, 90), 1e-4, "F32", 16, 100_000, 3_000),
+    (1, (200, 180), 1e-9, "F64", 1, 100_000, 2_000),
+    (2, (200, 180), 1e-9, "F64", 1, 300_000, 2_000),
+])
+def test_sparser_points_are_set_and_executed_in_a_graph(kind, n_modes, eps, precision, batch, many, few):
+    """A plan that has run on many points takes fewer inside a capture, where
+    nothing can be allocated, whichever kernels its rules choose for them."""
+    import torch
+
+    import wgpunufft_b200 as w
+
+    real, cplx = (torch.float32, torch.complex64) if precision == "F32" else (torch.float64, torch.complex128)
+    rng = np.random.default_rng(25)
+    total = int(np.prod(n_modes))
+    config = w.NufftConfig(n_modes, eps, batch=batch, precision=getattr(w.Precision, precision))
+
+    def buffers(count):
+        points = torch.from_numpy(rng.uniform(-np.pi, np.pi, (count, len(n_modes)))).to("cuda", real)
+        points.clamp_(-3.1415, 3.1415)
+        inputs = torch.from_numpy(values(rng, batch, count if kind == 1 else total)).to("cuda", cplx)
+        return points, inputs, torch.empty((batch, total if kind == 1 else count), dtype=cplx, device="cuda")
+
+    plan, stream = w.NufftPlan(kind, config), torch.cuda.Stream()
+    points, inputs, out = buffers(few)
+    with torch.cuda.stream(stream):
+        plan.encode_gpu(*buffers(many), stream=stream)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            plan.encode_gpu(points, inputs, out, stream=stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    captured = out.clone()
+    alone = w.NufftPlan(kind, config)
+    alone.encode_gpu(points, inputs, out)
+    alone.synchronize()
+    assert torch.equal(torch.view_as_real(captured), torch.view_as_real(out))
+    del graph

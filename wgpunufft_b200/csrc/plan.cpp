@@ -21,6 +21,11 @@ constexpr int64_t kMaxPoints = (int64_t(1) << 30) - 1;
 // Active batches from which 2D f32 type-2 plans stage bin regions in shared memory.
 constexpr int kInterpBinsMinBatch = 8;
 
+// Points from which plans that can take the 2D batched strips always do.
+constexpr int64_t kStripsAlways = 75'000;
+// Bins of the 3D gather's point order: one cell along y and z, 8 along x.
+constexpr int32_t kRowsShift[3] = {3, 0, 0};
+
 int64_t mode_for_storage_index(int order, int64_t index, int64_t length) {
   // src/direct.rs:120-131
   if (order == B200NUFFT_MODE_ORDER_CENTERED) return index - length / 2;
@@ -402,12 +407,6 @@ void NufftPlan::configure_type2_bins() {
 
 void NufftPlan::configure_tiles() {
   SpreadParams& sp = spread_;
-  int64_t kept_candidate_base[3];
-  int32_t kept_candidate_count[3];
-  for (int a = 0; a < 3; ++a) {
-    kept_candidate_base[a] = sp.candidate_base[a];
-    kept_candidate_count[a] = sp.candidate_count[a];
-  }
   std::memset(&sp, 0, sizeof(sp));
   sp.grid = grid_;
   const int w = kernel_.width;
@@ -416,9 +415,7 @@ void NufftPlan::configure_tiles() {
   // most 8 cells.
   tc_active_ = tc_enabled_ && grid_.axis[1].shift == 0 && grid_.axis[0].shift <= 3;
   const TileShape shape = tile_shape(grid_, f64, tc_active_, tuned_, point_count_);
-  int64_t tile[3];
   for (int a = 0; a < 3; ++a) {
-    tile[a] = shape.tile[a];
     sp.tile[a] = shape.tile[a];
     sp.pad[a] = shape.pad[a];
     sp.ntiles[a] = shape.ntiles[a];
@@ -464,29 +461,41 @@ void NufftPlan::configure_tiles() {
     sp.crowded_points = shape.crowded_points;
     sp.cap_bins = bins_;
   }
-  const int64_t part_bound = shape.part_bound;
+  FoldTable& table = fold_tables_[shape.regs64];
+  build_fold_table(shape, table);
+  for (int a = 0; a < dim_; ++a) {
+    sp.candidate_base[a] = table.base[a];
+    sp.candidate_count[a] = table.count[a];
+  }
+  sp.dest_fold = table.dest_fold;
+  part_upper_bound_ = shape.part_bound;
+  // A later, sparser set of a plan on register tiles takes the shared-memory
+  // tiles: what it needs is kept ready, so that it can be set where nothing can
+  // be allocated or copied (a graph capture).
+  tiles_reserved_ = shape.tile_count;
+  scratch_reserved_ = 0;
+  if (shape.regs64 != 0) {
+    const TileShape sparse = tile_shape(grid_, f64, false, tuned_, reg64_least_points(grid_) - 1);
+    build_fold_table(sparse, fold_tables_[0]);
+    tiles_reserved_ = std::max(tiles_reserved_, sparse.tile_count);
+    scratch_reserved_ = static_cast<size_t>(sparse.part_bound) * sparse.padded_cells * 2 * scalar_bytes();
+  }
+}
+
+void NufftPlan::build_fold_table(const TileShape& shape, FoldTable& table) {
   // Candidate (tile, local) pairs of every coordinate of every axis: tile t
   // covers cells (t * tile + l) mod n for l < pad. They depend on the grid
   // and tile shape only, so later point sets reuse them.
-  if (!host_candidates_.empty() && candidate_tile_[0] == tile[0] && candidate_tile_[1] == tile[1] &&
-      candidate_tile_[2] == tile[2]) {
-    for (int a = 0; a < 3; ++a) {
-      sp.candidate_base[a] = kept_candidate_base[a];
-      sp.candidate_count[a] = kept_candidate_count[a];
-    }
-    sp.dest_fold = dest_fold_;
-    part_upper_bound_ = part_bound;
-    return;
-  }
-  host_candidates_.clear();
-  for (int a = 0; a < 3; ++a) candidate_tile_[a] = tile[a];
-  bool dest_fold = dim_ == 3 && tile[0] == 16 && tile[1] == 16 && tile[2] % 4 == 0;
+  if (!table.host.empty() && std::equal(shape.tile, shape.tile + 3, table.tile)) return;
+  table.host.clear();
+  std::copy(shape.tile, shape.tile + 3, table.tile);
+  bool dest_fold = dim_ == 3 && shape.tile[0] == 16 && shape.tile[1] == 16 && shape.tile[2] % 4 == 0;
   for (int a = 0; a < dim_; ++a) {
     const int64_t n = fine_[a];
     std::vector<std::vector<int2>> lists(static_cast<size_t>(n));
-    for (int64_t t = 0; t < sp.ntiles[a]; ++t) {
-      for (int64_t l = 0; l < sp.pad[a]; ++l) {
-        const int64_t cell = (t * tile[a] + l) % n;
+    for (int64_t t = 0; t < shape.ntiles[a]; ++t) {
+      for (int64_t l = 0; l < shape.pad[a]; ++l) {
+        const int64_t cell = (t * int64_t{shape.tile[a]} + l) % n;
         lists[static_cast<size_t>(cell)].push_back(make_int2(static_cast<int>(t), static_cast<int>(l)));
       }
     }
@@ -496,10 +505,10 @@ void NufftPlan::configure_tiles() {
     // tile's first cell in their order: every cell of the tile must list an
     // ordered part of them, each tile once.
     dest_fold = dest_fold && most <= 2;
-    for (int64_t t = 0; dest_fold && t < sp.ntiles[a]; ++t) {
-      const auto& first = lists[static_cast<size_t>(t * tile[a])];
+    for (int64_t t = 0; dest_fold && t < shape.ntiles[a]; ++t) {
+      const auto& first = lists[static_cast<size_t>(t * int64_t{shape.tile[a]})];
       if (first.size() == 2 && first[0].x == first[1].x) dest_fold = false;
-      for (int64_t c = t * tile[a]; dest_fold && c < std::min<int64_t>((t + 1) * tile[a], n); ++c) {
+      for (int64_t c = t * int64_t{shape.tile[a]}; dest_fold && c < std::min<int64_t>((t + 1) * int64_t{shape.tile[a]}, n); ++c) {
         size_t at = 0;
         for (const int2& e : lists[static_cast<size_t>(c)]) {
           while (at < first.size() && first[at].x != e.x) ++at;
@@ -511,22 +520,19 @@ void NufftPlan::configure_tiles() {
         }
       }
     }
-    sp.candidate_base[a] = static_cast<int64_t>(host_candidates_.size());
-    sp.candidate_count[a] = static_cast<int32_t>(most);
+    table.base[a] = static_cast<int64_t>(table.host.size());
+    table.count[a] = static_cast<int32_t>(most);
     for (const auto& list : lists) {
       for (size_t k = 0; k < most; ++k) {
-        host_candidates_.push_back(k < list.size() ? list[k] : make_int2(-1, -1));
+        table.host.push_back(k < list.size() ? list[k] : make_int2(-1, -1));
       }
     }
   }
-  dest_fold_ = dest_fold ? 1 : 0;
-  sp.dest_fold = dest_fold_;
-  void* cand = candidates_.reserve(host_candidates_.size() * sizeof(int2), "fold candidates");
-  check_cuda(cudaMemcpy(cand, host_candidates_.data(), host_candidates_.size() * sizeof(int2),
+  table.dest_fold = dest_fold ? 1 : 0;
+  void* cand = table.device.reserve(table.host.size() * sizeof(int2), "fold candidates");
+  check_cuda(cudaMemcpy(cand, table.host.data(), table.host.size() * sizeof(int2),
                         cudaMemcpyHostToDevice),
              "upload fold candidates");
-  spread_.grid = grid_;
-  part_upper_bound_ = part_bound;
 }
 
 int NufftPlan::choose_geometry(int64_t point_count) const {
@@ -668,6 +674,9 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
       check_cuda(cudaMemcpyAsync(kept, order, static_cast<size_t>(count) * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                                  stream),
                  "keep strip order");
+      // (Where a later set of fewer points goes by the bins, in a graph capture.)
+      staged_.reserve(static_cast<size_t>(std::min<int64_t>(count, kStripsAlways)) * ((batch_ + 31) / 32 * 32) * sizeof(float2),
+                      "staged type-2 values");
       StageScope scope(&timer_, kStageBinOffsets, stream);
       prepare_windows(static_cast<const float*>(points), kept, count, grid_,
                       tc2_windows_.reserve(static_cast<size_t>(count) * prepared_window_bytes(dim_), "strip windows"),
@@ -679,7 +688,7 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
     if (rows_order_) {
       uint64_t stride = 0;
       const GridParams rows = rows_grid(&stride);
-      uint32_t* rows_offsets = static_cast<uint32_t*>(rows_offsets_.reserve((stride + 1) * sizeof(uint32_t),
+      uint32_t* rows_offsets = static_cast<uint32_t*>(rows_offsets_.reserve((rows_bins_reserved() + 1) * sizeof(uint32_t),
                                                                            "row-order offsets"));
       uint32_t* order = nullptr;
       uint32_t* keys = nullptr;
@@ -722,7 +731,7 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
     if (rows_order_) {
       uint64_t stride = 0;
       const GridParams rows = rows_grid(&stride);
-      uint32_t* rows_offsets = static_cast<uint32_t*>(rows_offsets_.reserve((stride + 1) * sizeof(uint32_t),
+      uint32_t* rows_offsets = static_cast<uint32_t*>(rows_offsets_.reserve((rows_bins_reserved() + 1) * sizeof(uint32_t),
                                                                            "row-order offsets"));
       uint32_t* order = nullptr;
       uint32_t* keys = nullptr;
@@ -738,8 +747,8 @@ void NufftPlan::set_points(int64_t count, const void* points, cudaStream_t strea
   }
   if (type_ == 1) {
     configure_tiles();
-    parts_.reserve(static_cast<size_t>(spread_.tile_count) * sizeof(uint32_t), "tile parts");
-    part_start_.reserve(static_cast<size_t>(spread_.tile_count + 1) * sizeof(uint32_t),
+    parts_.reserve(static_cast<size_t>(tiles_reserved_) * sizeof(uint32_t), "tile parts");
+    part_start_.reserve(static_cast<size_t>(tiles_reserved_ + 1) * sizeof(uint32_t),
                         "tile part offsets");
     spread_count_parts(spread_, offsets, static_cast<uint32_t*>(parts_.get()),
                        static_cast<uint32_t*>(part_start_.get()), stream, &timer_);
@@ -863,7 +872,7 @@ void NufftPlan::execute_f32(int batch, const void* input, void* output, uint64_t
       t.scratch = static_cast<float2*>(scratch_.reserve(static_cast<size_t>(tc_part_upper_bound_) * groups *
                                                             kTcVectors * spread_.padded_cells * sizeof(float2),
                                                         "spreading tiles"));
-      t.candidates = static_cast<const int2*>(candidates_.get());
+      t.candidates = candidates();
       t.fine = fine;
       t.error_flag = static_cast<uint32_t*>(counters_.get()) + 7;
       tc_spread_execute(spread_, t, stream, &timer_);
@@ -887,7 +896,7 @@ void NufftPlan::execute_f32(int batch, const void* input, void* output, uint64_t
     l.part_upper_bound = part_upper_bound_;
     l.max_bits = static_cast<uint32_t*>(max_bits_.get());
     l.scratch = static_cast<float2*>(scratch_.reserve(scratch_bytes, "spreading tiles"));
-    l.candidates = static_cast<const int2*>(candidates_.get());
+    l.candidates = candidates();
     l.fine = fine;
     l.valid_mask = static_cast<const uint32_t*>(valid_mask_.get());
     if (fused_fold(batch)) {
@@ -1038,8 +1047,8 @@ void NufftPlan::execute_f64(int batch, const void* input, void* output, uint64_t
       check_cuda(cudaMemsetAsync(output, 0, out_bytes, stream), "zero type-1 output");
       return;
     }
-    const size_t scratch_bytes = static_cast<size_t>(part_upper_bound_) * batch *
-                                 spread_.padded_cells * sizeof(double2);
+    const size_t scratch_bytes =
+        batch * std::max(static_cast<size_t>(part_upper_bound_) * spread_.padded_cells * sizeof(double2), scratch_reserved_);
     SpreadLaunch64 l;
     l.points = static_cast<const double*>(sorted_points_.get());
     l.strengths = in;
@@ -1051,7 +1060,7 @@ void NufftPlan::execute_f64(int batch, const void* input, void* output, uint64_t
     l.part_upper_bound = part_upper_bound_;
     l.max_bits = static_cast<unsigned long long*>(max_bits_.get());
     l.scratch = static_cast<double2*>(scratch_.reserve(scratch_bytes, "spreading tiles"));
-    l.candidates = static_cast<const int2*>(candidates_.get());
+    l.candidates = candidates();
     l.fine = fine;
     l.valid_mask = static_cast<const uint32_t*>(valid_mask_.get());
     spread_execute64(spread_, l, stream, &timer_);
@@ -1220,7 +1229,7 @@ void NufftPlan::spread_to(int64_t active_batch, const void* strengths, void* gri
     l.scratch = static_cast<float2*>(scratch_.reserve(
         static_cast<size_t>(part_upper_bound_) * batch * spread_.padded_cells * sizeof(float2),
         "spreading tiles"));
-    l.candidates = static_cast<const int2*>(candidates_.get());
+    l.candidates = candidates();
     l.fine = static_cast<float2*>(grid);
     l.valid_mask = static_cast<const uint32_t*>(valid_mask_.get());
     spread_execute(spread_, l, stream, &timer_);
@@ -1236,9 +1245,9 @@ void NufftPlan::spread_to(int64_t active_batch, const void* strengths, void* gri
     l.part_upper_bound = part_upper_bound_;
     l.max_bits = static_cast<unsigned long long*>(max_bits_.get());
     l.scratch = static_cast<double2*>(scratch_.reserve(
-        static_cast<size_t>(part_upper_bound_) * batch * spread_.padded_cells * sizeof(double2),
+        batch * std::max(static_cast<size_t>(part_upper_bound_) * spread_.padded_cells * sizeof(double2), scratch_reserved_),
         "spreading tiles"));
-    l.candidates = static_cast<const int2*>(candidates_.get());
+    l.candidates = candidates();
     l.fine = static_cast<double2*>(grid);
     l.valid_mask = static_cast<const uint32_t*>(valid_mask_.get());
     spread_execute64(spread_, l, stream, &timer_);
@@ -1267,6 +1276,7 @@ bool NufftPlan::strips_for_batch(int batch) const {
   if (batch < tc_min_batch_ || kernel_.width < 3) return false;
   if (kernel_.width >= 6) return point_count_ >= 3'000 || batch > 32;
   if (batch > 24) return false;
+  // (All of kStripsAlways points or more.)
   if (2 * point_count_ >= fine_count_ && point_count_ >= 3'000) return true;
   return fine_count_ >= 150'000 ? point_count_ >= 8'000 : batch <= 16 && point_count_ >= 16'000;
 }
@@ -1297,8 +1307,16 @@ GridParams NufftPlan::rows_grid(uint64_t* bins) const {
   // other 3D plans) bins of one cell along y and z and 8 cells along x: a
   // warp's 32 points then gather from few grid rows.
   if (interp_strips()) return strips_grid(bins);
-  const int32_t shift[3] = {3, 0, 0};
-  return bins_grid(shift, bins);
+  return bins_grid(kRowsShift, bins);
+}
+
+uint64_t NufftPlan::rows_bins_reserved() const {
+  // The larger of the two orders, either of which a later point set may take
+  // where nothing can be allocated (a graph capture).
+  uint64_t strips = 0, rows = 0;
+  strips_grid(&strips);
+  if (dim_ == 3) bins_grid(kRowsShift, &rows);
+  return std::max(strips, rows);
 }
 
 void NufftPlan::keep_rows_order(const uint32_t* order, int64_t count, cudaStream_t stream) {
@@ -1434,7 +1452,7 @@ void NufftPlan::finish_batch(void* output, cudaStream_t stream) {
   l.part_start = static_cast<const uint32_t*>(part_start_.get());
   l.part_upper_bound = part_upper_bound_;
   l.scratch = static_cast<float2*>(scratch_.get());
-  l.candidates = static_cast<const int2*>(candidates_.get());
+  l.candidates = candidates();
   l.fine = fine;
   if (fused_fold(1)) {
     float2* rows = static_cast<float2*>(

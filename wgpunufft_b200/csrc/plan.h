@@ -172,6 +172,7 @@ class NufftPlan {
   GridParams bins_grid(const int32_t sides_log2[3], uint64_t* bins) const;
   GridParams strips_grid(uint64_t* bins) const;
   GridParams rows_grid(uint64_t* bins) const;
+  uint64_t rows_bins_reserved() const;
   // Copies a sort's permutation into rows_perm_ (the sort buffers are reused).
   void keep_rows_order(const uint32_t* order, int64_t count, cudaStream_t stream);
   // The reference's bin order (perm_, offsets_, sorted_keys_) of a point set
@@ -183,13 +184,24 @@ class NufftPlan {
   SortBuffers sort_buffers(int64_t count);
 
   // Spreading state.
-  DeviceBuffer parts_, part_start_, max_bits_, scratch_, candidates_;
+  DeviceBuffer parts_, part_start_, max_bits_, scratch_;
   DeviceBuffer warp_segments_;     // 3D f32: segment table of the warp spreader
   int32_t warp_layout_key_[4] = {};  // width and padded tile of that table
   int64_t part_upper_bound_ = 0;
-  std::vector<int2> host_candidates_;
-  int64_t candidate_tile_[3] = {0, 0, 0};
-  int32_t dest_fold_ = 0;  // SpreadParams::dest_fold of the kept candidate table
+  // Fold candidates of a tile shape; the register tiles' (3D f64) and the others'.
+  struct FoldTable {
+    std::vector<int2> host;
+    int32_t tile[3] = {0, 0, 0};
+    int64_t base[3] = {0, 0, 0};
+    int32_t count[3] = {0, 0, 0};
+    int32_t dest_fold = 0;
+    DeviceBuffer device;
+  };
+  FoldTable fold_tables_[2];  // [SpreadParams::regs64]
+  void build_fold_table(const TileShape& shape, FoldTable& table);
+  const int2* candidates() const { return static_cast<const int2*>(fold_tables_[spread_.regs64].device.get()); }
+  int64_t tiles_reserved_ = 0;    // tiles that the part tables hold
+  size_t scratch_reserved_ = 0;   // scratch bytes per vector kept for sparser sets
 
   // Tensor-core spreading (2D f32 type-1 plans of batch >= kTcMinBatch):
   // enabled by the configuration, active when the chosen bins allow it.

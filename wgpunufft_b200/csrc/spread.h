@@ -84,6 +84,8 @@ struct TileShape {
 // and bin shifts).
 TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const b200nufft_tuning& tuning,
                      int64_t points);
+// Points from which 3D f64 plans of the register widths spread in registers.
+int64_t reg64_least_points(const GridParams& grid);
 // For tests: regs64, the tile's sides, tile count, padded cells, rows, part bound
 // and cap_parts under the default tuning.
 extern "C" int b200nufft_internal_tile_shape(int32_t dimensions, int32_t f64, int32_t width, const int64_t* fine,

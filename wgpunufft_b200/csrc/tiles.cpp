@@ -42,6 +42,11 @@ int64_t reg64_cells_per_point(int w) {
 
 }  // namespace
 
+int64_t reg64_least_points(const GridParams& grid) {
+  const int64_t per_point = reg64_cells_per_point(grid.width);
+  return (grid.fine_count + per_point - 1) / per_point;
+}
+
 TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const b200nufft_tuning& tuning,
                      int64_t points) {
   TileShape s{};
@@ -59,7 +64,7 @@ TileShape tile_shape(const GridParams& grid, bool f64, bool tensor_cores, const 
   }
   for (int a = 0; a < dim; ++a) tile[a] = std::min(tile[a], pow2_ceil(grid.fine[a]));
   const bool regs64 = dim == 3 && f64 && w >= kReg64MinWidth && w <= kReg64MaxWidth &&
-                      points * reg64_cells_per_point(w) >= grid.fine_count;
+                      points >= reg64_least_points(grid);
   auto padded_bytes = [&]() {
     int64_t cells = 1;
     for (int a = 0; a < dim; ++a) cells *= tile[a] + w - 1;
